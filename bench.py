@@ -42,30 +42,30 @@ WORKLOADS = {
 }
 METRIC = "seeds verified/s"
 UNIT = "seeds/s"
-# Algorithmic 32-bit integer operations per surviving seed (L = 4 limbs):
-# one k-step jump (4L) plus, per odd run, 3L + 2 (L shifts, L multiply-adds,
-# ctz, table, overflow test) and, per even run, 2L + 4 (decrement, ctz, L
-# shifts, increment with carry, descent test).
-OPS_JUMP, OPS_ODD, OPS_EVEN = 16, 14, 12
+# Algorithmic 32-bit integer operations per surviving seed with values of W words:
+# the step to the lane's next block (W adds), then per window W shifts, W
+# multiply-adds and 7 more (table index, the entry's three fields, the update and the
+# two tests of the coefficient).  Windows per seed: counted by a diagnostics build of
+# the kernel on the workload.
+OPS_WINDOW = 7
+WORK_MODEL = {"block": {"words": 2, "windows": 1.81}, "frontier": {"words": 3, "windows": 1.77}}
 # Counters of one range-kernel launch taken with ncu, valid only for the
 # sources of the kernel they were captured from: `src` is
 # kernel_source_hash(workload) at capture time (the kernel's own file and the
 # headers and table code it shares), and a line reports them only while those
 # sources still hash to it.
-#   block:    k_range64, 2^33 launch at 2^40, k = 24 (dram bytes per launch do
-#             not grow with the block: the 4.6 MB survivor table is read from
-#             DRAM once and from L2 after that);
-#   frontier: k_range, 2^36 launch at 2^60, k = 34 (dram bytes per 2^34 block:
-#             each block streams the 5 mod-9 classes it keeps of the 2.43 GB
-#             table).
+#   block:    k_range on two-word values, 2^34 launch at 2^40, k = 24 (dram bytes per
+#             launch do not grow with the block: the 4.6 MB survivor table is read
+#             from DRAM once and from L2 after that);
+#   frontier: k_range on three-word values, 2^36 launch at 2^60, k = 34.
 NCU_CAPTURES = {
-    "block": {"src": "212c53bc6b1ae53d", "dram_bytes": 5.210368e6 + 0.406272e6, "per": "launch",
-              "issue_slots_busy": 0.7923, "alu_pipe_busy": 0.6873, "kernel": "k_range64 (64-bit values)"},
-    "frontier": {"src": "756669d9f18f48b4", "dram_bytes": (5.423305e9 + 9.317888e6) / 4, "per": "2^34 block",
-                 "issue_slots_busy": 0.7581, "alu_pipe_busy": 0.6762, "kernel": "k_range (four limbs)"},
+    "block": {"src": "", "dram_bytes": 0, "per": "launch",
+              "issue_slots_busy": 0, "alu_pipe_busy": 0, "kernel": "k_range (two words)"},
+    "frontier": {"src": "", "dram_bytes": 0, "per": "launch",
+                 "issue_slots_busy": 0, "alu_pipe_busy": 0, "kernel": "k_range (three words)"},
 }
-SHARED_KERNEL_SOURCES = ("range_shared.cuh", "common.cuh", "kernels.h", "tables.h", "tables.cu")
-KERNEL_SOURCES = {"block": ("range64.cu",) + SHARED_KERNEL_SOURCES,
+SHARED_KERNEL_SOURCES = ("common.cuh", "kernels.h", "tables.h", "tables.cu")
+KERNEL_SOURCES = {"block": ("range.cu",) + SHARED_KERNEL_SOURCES,
                   "frontier": ("range.cu",) + SHARED_KERNEL_SOURCES}
 # CPU sample of the block workload, the same for the reference arm's steps and
 # the cpu_baseline leg: 2^32 seeds at 2^40 + i 2^32 with the k = 24 sieve.
@@ -508,16 +508,12 @@ def run_served(v, capacity: float, load: float = 0.7, duration: float = 1.0, see
 def roofline(workload: str, base: int, k: int, survivors: int, mean_ms: float, size: int, sm_count: int,
              sm_mhz: float, ipk: dict) -> dict:
     """Integer roofline of one k_range launch: algorithmic 32-bit operations
-    (per surviving seed: the jump plus the odd and even runs the oracle's
-    jump+runs model counts on a 2^24-seed sample of the same workload) per
-    second of device time, against the measured integer peak at the sampled
-    SM clock.  ncu counters are attached only while the kernel sources still
+    (WORK_MODEL) per second of device time, against the measured integer peak at the
+    sampled SM clock.  ncu counters are attached only while the kernel sources still
     hash to those they were captured from."""
-    from oracle import oracle as O
-    samp = O.range_verify(base, 1 << 24, k, True, 2, min(8, os.cpu_count() or 1))
-    odd_per = samp.odd_runs / samp.seeds
-    even_per = samp.even_runs / samp.seeds
-    ops_per_seed = OPS_JUMP + OPS_ODD * odd_per + OPS_EVEN * even_per
+    m = WORK_MODEL[workload]
+    ops_per_window = 2 * m["words"] + OPS_WINDOW
+    ops_per_seed = m["words"] + m["windows"] * ops_per_window
     achieved = survivors * ops_per_seed / (mean_ms / 1e3) / 1e12
     peak = ipk[1]["ops_per_clk_sm"] * sm_count * sm_mhz * 1e6 / 1e12
     issue_peak = sm_count * 128 * sm_mhz * 1e6 / 1e12
@@ -533,8 +529,8 @@ def roofline(workload: str, base: int, k: int, survivors: int, mean_ms: float, s
                            f"kernel sources {cap['src']}" + (f" x {max(1, size >> k)} blocks" if cap["per"] != "launch"
                                                              else "")) if valid else
          f"null: the kernel sources ({src}) changed since the last ncu capture ({cap['src']})",
-         "model": f"{ops_per_seed:.1f} algorithmic 32-bit ops per surviving seed ({OPS_JUMP} + {OPS_ODD} x "
-                  f"{odd_per:.2f} odd runs + {OPS_EVEN} x {even_per:.2f} even runs) x {survivors} seeds per launch",
+         "model": f"{ops_per_seed:.1f} algorithmic 32-bit ops per surviving seed ({m['words']} + {ops_per_window} x "
+                  f"{m['windows']} windows of 13 steps) x {survivors} seeds per launch",
          "peak_basis": f"measured integer peak (collatz_int_peak mix 1: funnel shift, 3-input add, multiply-add "
                        f"chains on every SM): {ipk[1]['ops_per_clk_sm']:.1f} ops per SM clock x {sm_count} SMs x "
                        f"{sm_mhz:.0f} MHz (sampled median SM clock); MEASURED_PEAKS.json has no integer peak",
@@ -824,7 +820,7 @@ def main():
             # 64-byte segments (5 kept mod-9 classes of the first and last block, 9 x 5 for the
             # blocks between), and the request's 4-byte first-segment index (threshold scouts)
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 32 + 64 * 55 + 4,
-                    "d2h_bytes_per_step": 136,
+                    "d2h_bytes_per_step": 144,
                     "call": "collatz_verify_range (lower + upload work list + launches + result copy)"},
             "clocks": clocks,
             # per step: k_range_scout, k_range and the two widening passes

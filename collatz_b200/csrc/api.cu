@@ -36,9 +36,9 @@ static void limbs4(u128 x, uint32_t* w) {
   for (int i = 0; i < 4; i++) w[i] = (uint32_t)(x >> (32 * i));
 }
 
-static int grid_for(collatz_ctx* c, int mode, int variant) {
+static int cases_grid(collatz_ctx* c, int variant) {
   int bps = 0;
-  cudaError_t e = mode == 0 ? cases_occupancy(variant, &bps) : range_occupancy(variant, &bps);
+  cudaError_t e = cases_occupancy(variant, &bps);
   if (e != cudaSuccess || bps <= 0) bps = 1;
   return bps * c->sm_count;
 }
@@ -282,8 +282,7 @@ extern "C" int collatz_create(const collatz_config* cfg, collatz_ctx** out) {
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking);
   for (int i = 0; i < 4 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
-  if (e == cudaSuccess) e = range_init();
-  if (e == cudaSuccess) e = range64_init();
+  if (e == cudaSuccess) e = range_init(c->own_stream);
   if (e == cudaSuccess) e = build_case_tables(&c->ct, cfg->maxbits, c->own_stream);
   if (e != cudaSuccess) {
     rc = set_cuda_error(c, e, "collatz_create");
@@ -456,7 +455,7 @@ extern "C" int collatz_verify_pairs(collatz_ctx* c, uint32_t bigindex, const uin
     CK(c, cudaMemsetAsync(c->d_counter.p, 0, sizeof(uint32_t), c->stream));
     CasesArgs a = case_args(c, c->d_pairs[0].as<uint32_t>(), npairs, (int)bigindex);
     CK(c, cudaEventRecord(c->ev[0], c->stream));
-    CK(c, launch_cases(a, c->cases_variant, grid_for(c, 0, c->cases_variant), c->stream));
+    CK(c, launch_cases(a, c->cases_variant, cases_grid(c, c->cases_variant), c->stream));
     CK(c, cudaEventRecord(c->ev[1], c->stream));
   }
   CK(c, cudaStreamSynchronize(c->stream));
@@ -656,7 +655,7 @@ static int run_case_host(collatz_ctx* c, const collatz_case* cs, collatz_case_re
       if (!err) err = cudaEventRecord(e0, c->stream);
       if (!err) {
         CasesArgs a = case_args(c, c->d_pairs[slot].as<uint32_t>(), job.second, -1);
-        err = launch_cases(a, c->cases_variant, grid_for(c, 0, c->cases_variant), c->stream);
+        err = launch_cases(a, c->cases_variant, cases_grid(c, c->cases_variant), c->stream);
       }
       if (!err) err = cudaEventRecord(e1, c->stream);
       if (!err) err = cudaEventRecord(kdone[slot], c->stream);
@@ -844,7 +843,7 @@ static int run_case_device(collatz_ctx* c, const collatz_case* cs, collatz_case_
       CK(c, s1_emit(c, R, lo, hi, dp));
       CK(c, cudaMemsetAsync(c->d_counter.p, 0, sizeof(uint32_t), c->stream));
       CasesArgs a = case_args(c, dp, (uint32_t)(hi - lo), -1);
-      CK(c, launch_cases(a, c->cases_variant, grid_for(c, 0, c->cases_variant), c->stream));
+      CK(c, launch_cases(a, c->cases_variant, cases_grid(c, c->cases_variant), c->stream));
     }
     CK(c, cudaEventRecord(c->ev[1], c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
@@ -1091,7 +1090,7 @@ static int range_lower_batch(collatz_ctx* c, const collatz_range* r, uint32_t n,
     const size_t before = segs.size();
     rc = lower_range(c, r[i], i, **T, segs, items);
     if (rc) return rc;
-    if (segs.size() > before) first_seg[i] = (uint32_t)before;  // the scouts' item
+    first_seg[i] = scout_segment(segs, before, items);
     *seed_bits = std::max(*seed_bits, range_seed_bits(r[i]));
   }
   if (segs.empty()) {  // keep the kernel's segment search well-defined
@@ -1140,19 +1139,12 @@ static RangeArgs range_args(collatz_ctx* c, const RangeTables& T, uint32_t k, bo
   return a;
 }
 
-cudaError_t cz::range_kernel_launch(collatz_ctx* c, const RangeArgs& a, bool stats, cudaStream_t s) {
-  if (!a.negative && a.seed_bits && a.seed_bits <= std::min(c->range64_bits, range64_max_seed_bits())) {
-    const int v = c->range64_variant;
-    int& bps = c->occ_range64[v & 7];
-    if (bps <= 0 && (range64_occupancy(v, &bps) != cudaSuccess || bps <= 0)) bps = 1;
-    const uint32_t grid = (uint32_t)(bps * c->sm_count);
-    return stats ? launch_range64_stats(a, v, grid, s) : launch_range64(a, v, grid, s);
-  }
-  const int v = c->range_variant;
-  int& bps = c->occ_range[v & 7];
-  if (bps <= 0 && (range_occupancy(v, &bps) != cudaSuccess || bps <= 0)) bps = 1;
-  const uint32_t grid = (uint32_t)(bps * c->sm_count);
-  return (stats && !a.negative) ? launch_range_stats(a, grid, s) : launch_range(a, v, grid, s);
+cudaError_t cz::range_kernel_launch(collatz_ctx* c, const RangeArgs& a, cudaStream_t s) {
+  const uint32_t bits = a.seed_bits ? a.seed_bits : 96;
+  const bool two = bits <= std::min(c->range64_bits, range64_max_seed_bits());
+  // three words hold 2^14 times a seed of 80 bits: few seeds outgrow them
+  const int words = two ? 2 : bits <= 80 ? 3 : 4;
+  return launch_range(a, words, two ? c->range64_variant : c->range_variant, (uint32_t)c->sm_count, s);
 }
 
 // One range launch on stream s: record and counter reset, k_range, the
@@ -1165,7 +1157,7 @@ static cudaError_t range_enqueue(collatz_ctx* c, const RangeArgs& a, const Range
   if (!e) e = cudaMemsetAsync(b.wcount, 0, sizeof(uint32_t) * 2, s);
   if (!e && b.stats) e = cudaMemsetAsync(b.stats, 0, 16 * sizeof(unsigned long long), s);
   if (!e && b.first_seg) e = launch_range_scout(a, b.first_seg, b.n, s);
-  if (!e) e = range_kernel_launch(c, a, b.stats != nullptr, s);
+  if (!e) e = range_kernel_launch(c, a, s);
   if (!e)
     e = launch_range_wide(b.widen, b.wcount, WIDEN_CAP, 6, b.recs, b.widen2, WIDEN_CAP, b.wcount + 1, c->iter_cap, s,
                           a.negative != 0);
@@ -1256,12 +1248,7 @@ extern "C" int collatz_plan_results(collatz_plan* p, collatz_range_result* out) 
   if (p->stats) {  // diagnostics (COLLATZ_RANGE_STATS=1)
     unsigned long long st8[16];
     CK(c, cudaMemcpy(st8, p->d_stats.p, sizeof st8, cudaMemcpyDeviceToHost));
-    fprintf(stderr,
-            "collatz range stats: run_pairs=%llu slow_e=%llu replays=%llu jumps=%llu pops=%llu expansions=%llu "
-            "passes=%llu offers=%llu windows=%llu pairs_64bit=%llu warp_cycles: offers=%llu refill=%llu "
-            "lanes=%llu (refill: wait=%llu stage=%llu thresholds=%llu)\n",
-            st8[0], st8[1], st8[2], st8[3], st8[4], st8[5], st8[6], st8[7], st8[14], st8[15], st8[8], st8[9],
-            st8[10], st8[11], st8[12], st8[13]);
+    fprintf(stderr, "collatz range stats: items=%llu runs=%llu exact_seeds=%llu\n", p->items, st8[0], st8[1]);
   }
   for (uint32_t i = 0; i < p->n; i++) {
     rec_to_range_result(h[i], &out[i]);

@@ -71,12 +71,13 @@ cudaError_t launch_step1_expand(const Step1Args& a, uint32_t bound, cudaStream_t
 cudaError_t launch_step1_walk(const Step1Args& a, bool emit, cudaStream_t st);
 
 // ---------------- range mode (range.cu) ----------------
-constexpr uint32_t RANGE_ITEM = 64;     // survivor-table entries per work item
+constexpr uint32_t RANGE_ITEM = 64;     // survivor-table entries per work item (a row)
 constexpr uint32_t DENSE_ITEM = 64;     // consecutive integers per dense work item
 
-// A run of work items of one request.  kind 0: survivor entries
-// [s_lo, s_hi) (one mod-9 class of the class-major table, or all of it) of
-// blocks q, q + qstride, ... (nq blocks; seeds n = q 2^k + r);
+// A segment of work items of one request.  kind 0: survivor entries
+// [s_lo, s_hi) of one mod-9 class of the class-major table, for
+// blocks q, q + qstride, ... (nq blocks; seeds n = q 2^k + r), item i being
+// entries s_lo + 64 (i / nq) onwards of block i mod nq;
 // kind 1: integers [d_lo, d_hi) iterated without the residue sieve.
 struct RangeSeg {
   unsigned long long item_begin;  // global index of the first item
@@ -89,8 +90,7 @@ struct RangeSeg {
   uint32_t req;                   // request index (ReqRec)
   uint16_t kind;
   uint16_t qstride;               // kind 0: block stride (0 or 1: consecutive blocks; 9: one q mod 9)
-  uint32_t mod9;                  // 1: apply the mod-9 sieve to each entry (0 when the segment's
-                                  //    classes are all kept by it)
+  uint32_t mod9;                  // kind 1: apply the mod-9 sieve (a kind 0 segment is a kept class)
   // Item index within the original segment of item_begin (non-zero when a
   // scheduler cuts a segment into slices; local indices stay < 2^32 for kind 0).
   uint32_t local0_lo, local0_hi;
@@ -114,44 +114,26 @@ struct RangeArgs {
   uint32_t* widen_count;
   uint32_t iter_cap;              // odd/even run pairs per seed before ERR_ITER_CAP
   uint32_t negative;              // 1: the negative-integer variant (a table built for it)
-  unsigned long long* stats;      // diagnostics counters (stats variant only), may be null
+  unsigned long long* stats;      // diagnostics: [0] runs of rows, [1] seeds on the exact path; may be null
   uint32_t seed_bits;             // bit length of the launch's largest seed (0: not known)
 };
-// Variants 4 and 5 run the 64-bit body (variants 6 and 7) when every seed of
-// the launch lies below 2^RANGE_NARROW_MAX_BITS: its values then stay below
-// 2^59 for most steps.  For seeds from 2^52 on, the 128-bit body alone is
-// faster (measured on B200: 2^34 seeds at 2^51 take 5.20 ms with the 64-bit
-// body and 5.21 ms without; at 2^52, 5.29 ms and 5.21 ms).
+// Cases mode: seeds below 2^52 run the 64-bit body (measured on the range kernel's
+// run loop: 2^34 seeds at 2^51 took 5.20 ms with it and 5.21 ms without; at 2^52,
+// 5.29 ms and 5.21 ms).
 constexpr uint32_t RANGE_NARROW_MAX_BITS = 52;
 int range_variants();
-cudaError_t range_init();  // once per device, before the first launch
-// Diagnostics variant (the default shape with 3 blocks per SM): counts run
-// pairs, slow paths, replays, jumps, pops, expansions, pop-block passes and
-// offers into a.stats[0..7], clock64 cycles per phase into [8..13], 8-step
-// windows taken into [14] and run pairs on the 64-bit body into [15].
-cudaError_t launch_range_stats(const RangeArgs& a, uint32_t grid, cudaStream_t st);
-cudaError_t launch_range(const RangeArgs& a, int variant, uint32_t grid, cudaStream_t st);
-cudaError_t range_occupancy(int variant, int* blocks_per_sm);
-// The 64-bit range kernel (range64.cu): the same seeds and results as
-// launch_range for launches of the positive variant whose seeds all lie
-// below 2^range64_max_seed_bits(); one 64-bit value per seed, four limbs per
-// lane only while a lane's value is at or above 2^59.  Variants differ in
-// run pairs per pass, resident blocks per SM and the in-loop table steps J
-// (0: none; 8, 10, 11).
 int range64_variants();
-// Hash of the 64-bit kernel's variant table (part of the autotuner's cache key).
-uint32_t range64_variant_rev();
+// Hash of the variant table (part of the autotuner's cache key).
+uint32_t range_variant_rev();
+// Launches whose seeds have at most this many bits may run on two-word values.
 uint32_t range64_max_seed_bits();
-cudaError_t range64_init();  // once per device, before the first launch
-cudaError_t launch_range64(const RangeArgs& a, int variant, uint32_t grid, cudaStream_t st);
-// Diagnostics form: run pairs, slow paths, replays, jumps, pops, expansions,
-// passes, offers into a.stats[0..7], table steps [13], windows [14], 64-bit
-// pairs [15]; clock64 cycles of offers, refill and lanes into [8..10].
-cudaError_t launch_range64_stats(const RangeArgs& a, int variant, uint32_t grid, cudaStream_t st);
-cudaError_t range64_occupancy(int variant, int* blocks_per_sm);
-// Threshold scouts: first_seg[i] is the index of request i's first segment
+cudaError_t range_init(cudaStream_t st);  // once per device, before the first launch; ends with st idle
+// The range kernel with values of 2, 3 or 4 words (a seed that outgrows them
+// takes the kernel's exact path, so any width gives the same results).
+cudaError_t launch_range(const RangeArgs& a, int words, int variant, uint32_t sm_count, cudaStream_t st);
+// Threshold scouts: first_seg[i] is the index of request i's scout segment
 // (>= a.nsegs: none).  Raises each request's prefilter keys to the maxima of
-// the seeds of its first work item, before the range kernel runs.
+// some of that segment's seeds, before the range kernel runs.
 cudaError_t launch_range_scout(const RangeArgs& a, const uint32_t* first_seg, uint32_t nreq, cudaStream_t st);
 // Seeds of a widen list re-run from scratch with 6 (then 8) limbs; the
 // list length is read on the device (*count, at most cap), so the pass can

@@ -37,7 +37,7 @@
 namespace cz {
 
 constexpr size_t NOALLOC_SCRATCH_BYTES = 64 * 1024;
-constexpr size_t NOALLOC_REC_OFF = 0;       // ReqRec (136 bytes)
+constexpr size_t NOALLOC_REC_OFF = 0;       // ReqRec (144 bytes)
 constexpr size_t NOALLOC_COUNTER_OFF = 256; // pair counter (u32)
 constexpr size_t NOALLOC_OVCOUNT_OFF = 264; // overflow count (u64)
 constexpr size_t NOALLOC_OVERFLOW_OFF = 512;

@@ -16,9 +16,9 @@ enum : uint32_t {
 };
 
 struct ReqRec {
-  unsigned long long seeds;       // seeds iterated
-  unsigned long long st_key;      // running max stopping time (prefilter)
+  unsigned long long st_key;      // running max stopping time (prefilter); with e_key one 16-byte copy
   unsigned long long e_key;       // monotone key of the running max excursion (prefilter)
+  unsigned long long seeds;       // seeds iterated
   unsigned long long failures;    // seeds that did not finish (beyond widest limbs / iteration cap)
   unsigned long long widened;     // seeds re-run with wider limbs
   unsigned long long items_done;  // work items completed (serving progress); cases line batches: overflow reports
@@ -30,7 +30,8 @@ struct ReqRec {
   uint32_t st_seed[4];            // its seed (smallest on ties)
   uint32_t E[8];                  // exact maximum excursion (little-endian limbs)
   uint32_t E_seed[4];             // its seed (smallest on ties)
+  uint32_t pad[2];                // records of an array stay 16-byte aligned
 };
-static_assert(sizeof(ReqRec) == 136, "ReqRec layout");
+static_assert(sizeof(ReqRec) == 144, "ReqRec layout");
 
 }  // namespace cz

@@ -113,12 +113,10 @@ struct collatz_ctx {
   cz::CaseTables ct;
   std::map<uint32_t, cz::RangeTables> rt;
   int cases_variant = 4, range_variant = 0;
-  // 64-bit range kernel: its variant, and the limb-width cutoff -- launches whose seeds
-  // all have at most range64_bits bits run it, the others run the four-limb kernel
+  // range kernel on two-word values: its variant, and the width cutoff -- launches whose
+  // seeds all have at most range64_bits bits run on two words, the others on three or four
   int range64_variant = 0;
   uint32_t range64_bits = 48;
-  // resident blocks per SM of each range-kernel variant (0: not asked yet)
-  int occ_range[8] = {}, occ_range64[8] = {};
   uint32_t iter_cap = 1u << 16;
   // scratch for the synchronous calls
   cz::DevBuf d_rec, d_counter, d_overflow, d_ovcount, d_pairs[2], d_segs, d_widen, d_widen2, d_wcount;
@@ -152,13 +150,26 @@ inline uint32_t range_seed_bits(const collatz_range& r) {
   return b;
 }
 int get_range_tables(collatz_ctx* c, uint32_t k, RangeTables** out, bool negative = false);
-// Launches the range kernel for a on stream s: the 64-bit kernel when every
-// seed of the launch has at most c->range64_bits bits (positive variant),
-// else the four-limb kernel; grid = resident blocks per SM x SMs.  stats:
-// the diagnostics form of the chosen kernel.
-cudaError_t range_kernel_launch(collatz_ctx* c, const RangeArgs& a, bool stats, cudaStream_t s);
+// Launches the range kernel for a on stream s, on two-word values when every
+// seed of the launch has at most c->range64_bits bits, on three up to 80 bits
+// and else on four.
+cudaError_t range_kernel_launch(collatz_ctx* c, const RangeArgs& a, cudaStream_t s);
 int lower_range(collatz_ctx* c, const collatz_range& r, uint32_t req, const RangeTables& T,
                 std::vector<RangeSeg>& segs, unsigned long long& items);
+// The segment of segs[from..) with the most items (items: the end of the last one), from
+// which a request's scouts are taken; ~0u when there is none.
+inline uint32_t scout_segment(const std::vector<RangeSeg>& segs, size_t from, unsigned long long items) {
+  uint32_t best = ~0u;
+  unsigned long long most = 0;
+  for (size_t i = from; i < segs.size(); i++) {
+    const unsigned long long n = (i + 1 < segs.size() ? segs[i + 1].item_begin : items) - segs[i].item_begin;
+    if (n > most) {
+      most = n;
+      best = (uint32_t)i;
+    }
+  }
+  return best;
+}
 void rec_to_range_result(const ReqRec& r, collatz_range_result* out);
 // Applies cached autotuner choices to a new context (tune.cu).
 void tune_on_create(collatz_ctx* c);

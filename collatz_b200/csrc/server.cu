@@ -132,7 +132,7 @@ __global__ void k_slice_prologue(unsigned long long* cursor, uint32_t* wcount, R
     wcount[0] = 0;
     wcount[1] = 0;
   }
-  constexpr uint32_t W = sizeof(ReqRec) / 8;  // 17 words of 8 bytes
+  constexpr uint32_t W = sizeof(ReqRec) / 8;  // 18 words of 8 bytes
   for (uint32_t i = t; i < nslots * W; i += gridDim.x * blockDim.x)
     reinterpret_cast<unsigned long long*>(recs + slots[i / W])[i % W] = 0ull;
 }
@@ -444,7 +444,7 @@ int launch_slice(collatz_server* s, int si) {
   std::vector<RangeSeg> segs;
   unsigned long long slice_items = 0, budget = s->cfg.slice_items;
   uint32_t seed_bits = 0;
-  std::vector<uint32_t> scouts;  // the first segment of each request that starts in this slice
+  std::vector<uint32_t> scouts;  // the scouts' segment of each request that starts in this slice
   for (size_t i = 0; i < want.size(); i++) {
     const unsigned long long share = std::max<unsigned long long>(1, budget / (want.size() - i));
     const unsigned long long q = std::min(want[i].first, share);
@@ -452,7 +452,7 @@ int launch_slice(collatz_server* s, int si) {
     const bool starts = want[i].second->cursor == 0;
     const size_t before = segs.size();
     take_items(want[i].second, q, segs, slice_items);
-    if (starts && segs.size() > before) scouts.push_back((uint32_t)before);
+    if (starts && segs.size() > before) scouts.push_back(scout_segment(segs, before, slice_items));
     budget -= std::min(budget, q);
     if (want[i].second->cursor == want[i].second->items) S.finishing.push_back(want[i].second);
   }
@@ -502,7 +502,7 @@ int launch_slice(collatz_server* s, int si) {
   if (!e && fb)
     e = launch_range_scout(a, reinterpret_cast<const uint32_t*>(static_cast<const char*>(S.d_segs.p) + sb),
                            (uint32_t)scouts.size(), st);
-  if (!e) e = range_kernel_launch(c, a, false, st);
+  if (!e) e = range_kernel_launch(c, a, st);
   if (!e)
     e = launch_range_wide(S.d_widen[0].as<WidenEntry>(), S.d_wcount.as<uint32_t>(), WIDEN_CAP, 6, a.recs,
                           S.d_widen[1].as<WidenEntry>(), WIDEN_CAP, S.d_wcount.as<uint32_t>() + 1, c->iter_cap, st,

@@ -40,7 +40,7 @@ std::string device_key(const collatz_ctx* c) {
   std::ostringstream k;
   k << name << ":sm" << p.multiProcessorCount << ":cc" << p.major << "." << p.minor << ":abi"
     << COLLATZ_ABI_VERSION << ":v" << range_variants() << "." << cases_variants() << "." << range64_variants()
-    << "." << std::hex << range64_variant_rev();
+    << "." << std::hex << range_variant_rev();
   return k.str();
 }
 
