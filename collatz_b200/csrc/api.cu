@@ -148,9 +148,8 @@ int lower_range(collatz_ctx* c, const collatz_range& r, uint32_t req, const Rang
   // 9), and with the mod-9 sieve a block keeps exactly the classes c with
   // (q 2^k + c) mod 9 in {0,1,3,6,7}: 5 of the 9, depending only on q mod 9.
   // So each emitted segment covers one whole class (or, in a partial first
-  // or last block, the class's residues in range), and every entry it names
-  // is a seed.  Blocks strictly between the first and the last are grouped
-  // by q mod 9 into segments with block stride 9.
+  // or last block, the class's residues in range) over the blocks that keep it,
+  // and every entry it names is a seed.
   const u128 lo = std::max(O, K);
   if (lo >= E) return COLLATZ_OK;
   const u128 qa = lo >> k, qb = (E - 1) >> k;
@@ -158,10 +157,10 @@ int lower_range(collatz_ctx* c, const collatz_range& r, uint32_t req, const Rang
   auto live = [&](u128 q, uint32_t cl) {
     return !mod9 || ((keep9 >> (((uint32_t)(q % 9) * k9 + cl) % 9)) & 1u);
   };
-  auto add = [&](u128 q, u128 nq, uint32_t stride, uint32_t s_lo, uint32_t s_hi) {
+  auto add = [&](u128 q, u128 nq, uint32_t stride, uint32_t cl, uint32_t s_lo, uint32_t s_hi) {
     if (s_lo >= s_hi || nq == 0) return;
     const uint32_t ipq = (s_hi - s_lo + RANGE_ITEM - 1) / RANGE_ITEM;
-    const u128 max_nq = std::max<uint32_t>(1u, 0xFFFFFFFFu / ipq);  // < 2^32 items per segment
+    const u128 max_nq = std::max<uint32_t>(5u, 0xFFFFFFFFu / ipq / 5u * 5u);  // < 2^32 items per segment
     while (nq > 0) {
       const uint32_t take = (uint32_t)std::min(nq, max_nq);
       RangeSeg g{};
@@ -175,10 +174,10 @@ int lower_range(collatz_ctx* c, const collatz_range& r, uint32_t req, const Rang
       g.req = req;
       g.kind = 0;
       g.qstride = (uint16_t)stride;
-      g.mod9 = 0;  // every class of the segment is kept
+      g.mod9 = cl;
       segs.push_back(g);
       items += (unsigned long long)take * ipq;
-      q += (u128)take * stride;
+      q += stride == 9 ? (u128)(take / 5) * 9 : (u128)take;  // (take is a multiple of 5 unless it is the last)
       nq -= take;
     }
   };
@@ -190,7 +189,7 @@ int lower_range(collatz_ctx* c, const collatz_range& r, uint32_t req, const Rang
       int rc = lower_bound_res(c, T, cl, r0, &a);
       if (!rc) rc = lower_bound_res(c, T, cl, r1, &b);
       if (rc) return rc;
-      add(q, 1, 1, a, b);
+      add(q, 1, 1, cl, a, b);
     }
     return COLLATZ_OK;
   };
@@ -200,14 +199,22 @@ int lower_range(collatz_ctx* c, const collatz_range& r, uint32_t req, const Rang
   if (rc) return rc;
   const u128 m0 = qa + 1, nm = qb - qa - 1;  // whole blocks in between
   if (nm > 0) {
-    if (!mod9) {
-      for (uint32_t cl = 0; cl < 9; cl++) add(m0, nm, 1, (uint32_t)T.dev.cls[cl], (uint32_t)T.dev.cls[cl + 1]);
-    } else {
-      for (uint32_t t = 0; t < 9 && (u128)t < nm; t++) {
-        const u128 qt = m0 + t, nt = (nm - t + 8) / 9;  // blocks m0 + t, m0 + t + 9, ...
-        for (uint32_t cl = 0; cl < 9; cl++)
-          if (live(qt, cl)) add(qt, nt, 9, (uint32_t)T.dev.cls[cl], (uint32_t)T.dev.cls[cl + 1]);
+    for (uint32_t cl = 0; cl < 9; cl++) {
+      if (!mod9) {
+        add(m0, nm, 1, cl, (uint32_t)T.dev.cls[cl], (uint32_t)T.dev.cls[cl + 1]);
+        continue;
       }
+      u128 first = 0, kept = nm / 9 * 5;  // 5 of any 9 consecutive blocks keep the class
+      uint32_t in_rest = 0;
+      bool any = false;
+      for (uint32_t t = 0; t < 9; t++) {
+        if (!live(m0 + t, cl)) continue;
+        if (!any) first = m0 + t;
+        any = true;
+        if ((u128)t < nm % 9) in_rest++;
+      }
+      kept += in_rest;
+      add(first, kept, 9, cl, (uint32_t)T.dev.cls[cl], (uint32_t)T.dev.cls[cl + 1]);
     }
   }
   return partial(qb, 0, rb);
@@ -303,10 +310,10 @@ extern "C" void collatz_destroy(collatz_ctx* c) {
   free_case_tables(&c->ct);
   for (auto& kv : c->rt) free_range_table(&kv.second.dev);
   DevBuf* bufs[] = {&c->d_rec, &c->d_counter, &c->d_overflow, &c->d_ovcount, &c->d_pairs[0], &c->d_pairs[1],
-                    &c->d_segs, &c->d_widen, &c->d_widen2, &c->d_wcount, &c->t_seeds, &c->t_st, &c->t_exc,
+                    &c->d_segs, &c->d_lists, &c->t_seeds, &c->t_st, &c->t_exc,
                     &c->t_status, &c->t_idx[0], &c->t_idx[1], &c->t_cnt, &c->s1_front[0], &c->s1_front[1],
                     &c->s1_off, &c->s1_cnt, &c->s1_scal, &c->s1_stk_num, &c->s1_stk_meta, &c->s1_hist, &c->d_recs,
-                    &c->d_rcursor, &c->d_first};
+                    &c->d_range};
   for (DevBuf* b : bufs) b->release();
   c->h_rec.release();
   c->h_pairs.release();
@@ -1063,7 +1070,7 @@ struct collatz_plan {
   RangeTables* T = nullptr;
   std::vector<RangeSeg> segs;
   unsigned long long items = 0;
-  DevBuf d_segs, d_recs, d_cursor, d_widen, d_widen2, d_wcount, d_stats, d_first;
+  DevBuf d_segs, d_range, d_lists, d_stats;  // d_range: head, then records
   HostBuf h_recs;
   bool stats = false, negative = false;
   cudaGraph_t graph = nullptr;
@@ -1075,7 +1082,7 @@ struct collatz_plan {
 // tables and lowers every request into segments.
 static int range_lower_batch(collatz_ctx* c, const collatz_range* r, uint32_t n, RangeTables** T, uint32_t* k_out,
                              bool* neg_out, std::vector<RangeSeg>& segs, unsigned long long& items,
-                             uint32_t* seed_bits, std::vector<uint32_t>& first_seg) {
+                             uint32_t* seed_bits) {
   const uint32_t k = r[0].k ? r[0].k : c->cfg.range_k;
   const bool neg = (r[0].flags & COLLATZ_RANGE_NEGATIVE) != 0;
   for (uint32_t i = 0; i < n; i++)  // one sieve (k, sign) per launch
@@ -1085,12 +1092,9 @@ static int range_lower_batch(collatz_ctx* c, const collatz_range* r, uint32_t n,
   int rc = get_range_tables(c, k, T, neg);
   if (rc) return rc;
   *seed_bits = 0;
-  first_seg.assign(n, ~0u);
   for (uint32_t i = 0; i < n; i++) {
-    const size_t before = segs.size();
     rc = lower_range(c, r[i], i, **T, segs, items);
     if (rc) return rc;
-    first_seg[i] = scout_segment(segs, before, items);
     *seed_bits = std::max(*seed_bits, range_seed_bits(r[i]));
   }
   if (segs.empty()) {  // keep the kernel's segment search well-defined
@@ -1108,15 +1112,12 @@ struct RangeBufs {
   RangeSeg* segs;
   uint32_t nsegs;
   unsigned long long items;
-  ReqRec* recs;
-  void* h_recs;  // pinned: the records come back here
+  RangeHead* head;  // followed by the n records
+  void* h_recs;     // pinned: the records come back here
   uint32_t n;
-  unsigned long long* cursor;
-  WidenEntry* widen;
-  WidenEntry* widen2;
-  uint32_t* wcount;  // 2 counters
+  RangeLists* lists;
   unsigned long long* stats;
-  const uint32_t* first_seg;  // per request: its first segment (threshold scouts)
+  ReqRec* recs() const { return reinterpret_cast<ReqRec*>(head + 1); }
 };
 
 static RangeArgs range_args(collatz_ctx* c, const RangeTables& T, uint32_t k, bool neg, const RangeBufs& b,
@@ -1127,12 +1128,10 @@ static RangeArgs range_args(collatz_ctx* c, const RangeTables& T, uint32_t k, bo
   a.k = k;
   a.segs = b.segs;
   a.nsegs = b.nsegs;
-  a.item_cursor = b.cursor;
   a.item_limit = b.items;
-  a.recs = b.recs;
-  a.widen = b.widen;
-  a.widen_cap = WIDEN_CAP;
-  a.widen_count = b.wcount;
+  a.head = b.head;
+  a.lists = b.lists;
+  a.recs = b.recs();
   a.iter_cap = c->iter_cap;
   a.stats = b.stats;
   a.negative = neg ? 1u : 0u;
@@ -1147,24 +1146,16 @@ cudaError_t cz::range_kernel_launch(collatz_ctx* c, const RangeArgs& a, cudaStre
   return launch_range(a, words, two ? c->range64_variant : c->range_variant, (uint32_t)c->sm_count, s);
 }
 
-// One range launch on stream s: record and counter reset, k_range, the
-// 192- and 256-bit widening passes, the record copy-back.  Captured into a
+// One range launch on stream s: head and record reset, k_range, the
+// candidates and wide seeds, the record copy-back.  Captured into a
 // graph by plans; issued directly by collatz_verify_batch.
 static cudaError_t range_enqueue(collatz_ctx* c, const RangeArgs& a, const RangeBufs& b, cudaStream_t s) {
   const size_t rb = sizeof(ReqRec) * std::max(1u, b.n);
-  cudaError_t e = cudaMemsetAsync(b.recs, 0, rb, s);
-  if (!e) e = cudaMemsetAsync(b.cursor, 0, sizeof(unsigned long long), s);
-  if (!e) e = cudaMemsetAsync(b.wcount, 0, sizeof(uint32_t) * 2, s);
+  cudaError_t e = cudaMemsetAsync(b.head, 0, sizeof(RangeHead) + rb, s);
   if (!e && b.stats) e = cudaMemsetAsync(b.stats, 0, 16 * sizeof(unsigned long long), s);
-  if (!e && b.first_seg) e = launch_range_scout(a, b.first_seg, b.n, s);
   if (!e) e = range_kernel_launch(c, a, s);
-  if (!e)
-    e = launch_range_wide(b.widen, b.wcount, WIDEN_CAP, 6, b.recs, b.widen2, WIDEN_CAP, b.wcount + 1, c->iter_cap, s,
-                          a.negative != 0);
-  if (!e)
-    e = launch_range_wide(b.widen2, b.wcount + 1, WIDEN_CAP, 8, b.recs, nullptr, 0, nullptr, c->iter_cap, s,
-                          a.negative != 0);
-  if (!e) e = cudaMemcpyAsync(b.h_recs, b.recs, rb, cudaMemcpyDeviceToHost, s);
+  if (!e) e = launch_range_finish(a, s);
+  if (!e) e = cudaMemcpyAsync(b.h_recs, b.recs(), rb, cudaMemcpyDeviceToHost, s);
   return e;
 }
 
@@ -1175,26 +1166,19 @@ static bool range_stats_requested() {
 
 static int plan_build(collatz_ctx* c, const collatz_range* r, uint32_t n, collatz_plan* p) {
   uint32_t k = 0, seed_bits = 0;
-  std::vector<uint32_t> first_seg;
-  int rc = range_lower_batch(c, r, n, &p->T, &k, &p->negative, p->segs, p->items, &seed_bits, first_seg);
+  int rc = range_lower_batch(c, r, n, &p->T, &k, &p->negative, p->segs, p->items, &seed_bits);
   if (rc) return rc;
   p->n = n;
   CK(c, p->d_segs.ensure(sizeof(RangeSeg) * p->segs.size()));
   CK(c, cudaMemcpy(p->d_segs.p, p->segs.data(), sizeof(RangeSeg) * p->segs.size(), cudaMemcpyHostToDevice));
-  CK(c, p->d_first.ensure(sizeof(uint32_t) * n));
-  CK(c, cudaMemcpy(p->d_first.p, first_seg.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice));
-  CK(c, p->d_recs.ensure(sizeof(ReqRec) * std::max(1u, n)));
+  CK(c, p->d_range.ensure(sizeof(RangeHead) + sizeof(ReqRec) * std::max(1u, n)));
   CK(c, p->h_recs.ensure(sizeof(ReqRec) * std::max(1u, n)));
-  CK(c, p->d_cursor.ensure(sizeof(unsigned long long)));
-  CK(c, p->d_widen.ensure(sizeof(WidenEntry) * WIDEN_CAP));
-  CK(c, p->d_widen2.ensure(sizeof(WidenEntry) * WIDEN_CAP));
-  CK(c, p->d_wcount.ensure(sizeof(uint32_t) * 2));
+  CK(c, p->d_lists.ensure(sizeof(RangeLists)));
   p->stats = range_stats_requested();
   if (p->stats) CK(c, p->d_stats.ensure(16 * sizeof(unsigned long long)));
-  const RangeBufs b{p->d_segs.as<RangeSeg>(), (uint32_t)p->segs.size(), p->items, p->d_recs.as<ReqRec>(),
-                    p->h_recs.p, n, p->d_cursor.as<unsigned long long>(), p->d_widen.as<WidenEntry>(),
-                    p->d_widen2.as<WidenEntry>(), p->d_wcount.as<uint32_t>(),
-                    p->stats ? p->d_stats.as<unsigned long long>() : nullptr, p->d_first.as<uint32_t>()};
+  const RangeBufs b{p->d_segs.as<RangeSeg>(), (uint32_t)p->segs.size(), p->items, p->d_range.as<RangeHead>(),
+                    p->h_recs.p, n, p->d_lists.as<RangeLists>(),
+                    p->stats ? p->d_stats.as<unsigned long long>() : nullptr};
   const RangeArgs a = range_args(c, *p->T, k, p->negative, b, seed_bits);
   cudaStream_t s = c->own_stream;
   CK(c, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
@@ -1264,13 +1248,9 @@ extern "C" void collatz_plan_destroy(collatz_plan* p) {
   if (p->exec) cudaGraphExecDestroy(p->exec);
   if (p->graph) cudaGraphDestroy(p->graph);
   p->d_segs.release();
-  p->d_recs.release();
-  p->d_cursor.release();
-  p->d_widen.release();
-  p->d_widen2.release();
-  p->d_wcount.release();
+  p->d_range.release();
+  p->d_lists.release();
   p->d_stats.release();
-  p->d_first.release();
   p->h_recs.release();
   delete p;
 }
@@ -1298,27 +1278,19 @@ extern "C" int collatz_verify_batch(collatz_ctx* c, const collatz_range* r, uint
   RangeTables* T = nullptr;
   uint32_t k = 0, seed_bits = 0;
   bool neg = false;
-  std::vector<uint32_t> first_seg;
-  int rc = range_lower_batch(c, r, n, &T, &k, &neg, segs, items, &seed_bits, first_seg);
+  int rc = range_lower_batch(c, r, n, &T, &k, &neg, segs, items, &seed_bits);
   if (rc) return rc;
-  const size_t sb = sizeof(RangeSeg) * segs.size(), rb = sizeof(ReqRec) * n, fb = sizeof(uint32_t) * n;
+  const size_t sb = sizeof(RangeSeg) * segs.size(), rb = sizeof(ReqRec) * n;
   CK(c, c->d_segs.ensure(sb));
-  CK(c, c->d_first.ensure(fb));
-  CK(c, c->h_segs.ensure(sb + fb));  // the segments, then the scouts' first segments
-  CK(c, c->d_recs.ensure(rb));
+  CK(c, c->h_segs.ensure(sb));
+  CK(c, c->d_range.ensure(sizeof(RangeHead) + rb));
   CK(c, c->h_recs.ensure(rb));
-  CK(c, c->d_rcursor.ensure(sizeof(unsigned long long)));
-  CK(c, c->d_widen.ensure(sizeof(WidenEntry) * WIDEN_CAP));
-  CK(c, c->d_widen2.ensure(sizeof(WidenEntry) * WIDEN_CAP));
-  CK(c, c->d_wcount.ensure(sizeof(uint32_t) * 2));
+  CK(c, c->d_lists.ensure(sizeof(RangeLists)));
   std::memcpy(c->h_segs.p, segs.data(), sb);
-  std::memcpy(static_cast<char*>(c->h_segs.p) + sb, first_seg.data(), fb);
-  const RangeBufs b{c->d_segs.as<RangeSeg>(), (uint32_t)segs.size(), items, c->d_recs.as<ReqRec>(), c->h_recs.p, n,
-                    c->d_rcursor.as<unsigned long long>(), c->d_widen.as<WidenEntry>(),
-                    c->d_widen2.as<WidenEntry>(), c->d_wcount.as<uint32_t>(), nullptr, c->d_first.as<uint32_t>()};
+  const RangeBufs b{c->d_segs.as<RangeSeg>(), (uint32_t)segs.size(), items, c->d_range.as<RangeHead>(), c->h_recs.p, n,
+                    c->d_lists.as<RangeLists>(), nullptr};
   const RangeArgs a = range_args(c, *T, k, neg, b, seed_bits);
   CK(c, cudaMemcpyAsync(c->d_segs.p, c->h_segs.p, sb, cudaMemcpyHostToDevice, c->stream));
-  CK(c, cudaMemcpyAsync(c->d_first.p, static_cast<char*>(c->h_segs.p) + sb, fb, cudaMemcpyHostToDevice, c->stream));
   CK(c, cudaEventRecord(c->ev[2], c->stream));
   CK(c, range_enqueue(c, a, b, c->stream));
   CK(c, cudaEventRecord(c->ev[3], c->stream));

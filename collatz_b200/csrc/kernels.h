@@ -76,8 +76,9 @@ constexpr uint32_t DENSE_ITEM = 64;     // consecutive integers per dense work i
 
 // A segment of work items of one request.  kind 0: survivor entries
 // [s_lo, s_hi) of one mod-9 class of the class-major table, for
-// blocks q, q + qstride, ... (nq blocks; seeds n = q 2^k + r), item i being
-// entries s_lo + 64 (i / nq) onwards of block i mod nq;
+// nq blocks from q on (seeds n = q 2^k + r): consecutive ones, or (qstride 9)
+// those that keep the class under the mod-9 sieve; item i is entries s_lo +
+// 64 (i / nq) onwards of the (i mod nq)-th block;
 // kind 1: integers [d_lo, d_hi) iterated without the residue sieve.
 struct RangeSeg {
   unsigned long long item_begin;  // global index of the first item
@@ -89,8 +90,8 @@ struct RangeSeg {
   uint32_t ipq;                   // kind 0: items per block
   uint32_t req;                   // request index (ReqRec)
   uint16_t kind;
-  uint16_t qstride;               // kind 0: block stride (0 or 1: consecutive blocks; 9: one q mod 9)
-  uint32_t mod9;                  // kind 1: apply the mod-9 sieve (a kind 0 segment is a kept class)
+  uint16_t qstride;               // kind 0: 0 or 1: consecutive blocks; 9: the blocks that keep the class
+  uint32_t mod9;                  // kind 0: the class (r mod 9); kind 1: 1 to apply the mod-9 sieve
   // Item index within the original segment of item_begin (non-zero when a
   // scheduler cuts a segment into slices; local indices stay < 2^32 for kind 0).
   uint32_t local0_lo, local0_hi;
@@ -101,21 +102,44 @@ struct WidenEntry {  // a seed to re-run with wider limbs
   uint32_t req, n0, n1, n2;
 };
 
+// A seed that may be its request's maximum stopping time (kind 0) or excursion (kind 1).
+struct RangeCand {
+  uint32_t req, kind, st, pad;
+  uint32_t E[4];
+  uint32_t seed[4];
+};
+static_assert(sizeof(RangeCand) == 48, "RangeCand");
+
+// Counters of a launch, zero before it.
+struct RangeHead {
+  unsigned long long item_cursor;  // next item to claim
+  uint32_t widened, cands;         // entries of the widen list and of the candidate list
+  uint32_t pad[12];
+};
+static_assert(sizeof(RangeHead) == 64, "RangeHead");
+
+// Lists of a launch; their lengths are in the head.
+constexpr uint32_t WIDEN_CAP = 1u << 16;
+constexpr uint32_t CAND_CAP = 1u << 15;  // candidates beyond it take the record's lock in the kernel
+struct RangeLists {
+  RangeCand cand[CAND_CAP];
+  WidenEntry widen[WIDEN_CAP];
+};
+
 struct RangeArgs {
   const RangeEntry* table;        // survivor table of the 2^k sieve
   uint32_t k;
   const RangeSeg* segs;
   uint32_t nsegs;
-  unsigned long long* item_cursor;  // scratch: next item to claim
   unsigned long long item_limit;    // items >= limit are not claimed in this launch
+  RangeHead* head;
+  RangeLists* lists;
   ReqRec* recs;
-  WidenEntry* widen;
-  uint32_t widen_cap;
-  uint32_t* widen_count;
   uint32_t iter_cap;              // odd/even run pairs per seed before ERR_ITER_CAP
   uint32_t negative;              // 1: the negative-integer variant (a table built for it)
   unsigned long long* stats;      // diagnostics: [0] runs of rows, [1] seeds on the exact path; may be null
   uint32_t seed_bits;             // bit length of the launch's largest seed (0: not known)
+  uint32_t one = 1, mone = ~0u, eight = 8;  // 1, -1 and 8, unknown to the compiler (range.cu: window)
 };
 // Cases mode: seeds below 2^52 run the 64-bit body (measured on the range kernel's
 // run loop: 2^34 seeds at 2^51 took 5.20 ms with it and 5.21 ms without; at 2^52,
@@ -131,16 +155,10 @@ cudaError_t range_init(cudaStream_t st);  // once per device, before the first l
 // The range kernel with values of 2, 3 or 4 words (a seed that outgrows them
 // takes the kernel's exact path, so any width gives the same results).
 cudaError_t launch_range(const RangeArgs& a, int words, int variant, uint32_t sm_count, cudaStream_t st);
-// Threshold scouts: first_seg[i] is the index of request i's scout segment
-// (>= a.nsegs: none).  Raises each request's prefilter keys to the maxima of
-// some of that segment's seeds, before the range kernel runs.
-cudaError_t launch_range_scout(const RangeArgs& a, const uint32_t* first_seg, uint32_t nreq, cudaStream_t st);
-// Seeds of a widen list re-run from scratch with 6 (then 8) limbs; the
-// list length is read on the device (*count, at most cap), so the pass can
-// sit in a captured graph right behind the range kernel.
-cudaError_t launch_range_wide(const WidenEntry* list, const uint32_t* count, uint32_t cap, int limbs,
-                              ReqRec* recs, WidenEntry* next, uint32_t next_cap, uint32_t* next_count,
-                              uint32_t iter_cap, cudaStream_t st, bool negative = false);
+// After the range kernel: the candidates into the records, and the widened seeds re-run
+// from scratch with 6 and then 8 limbs.  The list lengths are read on the device, so the
+// launch can sit in a captured graph.
+cudaError_t launch_range_finish(const RangeArgs& a, cudaStream_t st);
 
 // ---------------- trajectory queries (traj.cu) ----------------
 // All limb classes in one launch (traj.cu): index = the seed ids sorted by

@@ -95,7 +95,6 @@ inline std::string hex_u32(uint32_t x) {
   return s;
 }
 
-constexpr uint32_t WIDEN_CAP = 1u << 16;
 constexpr uint32_t OVERFLOW_CAP = 1u << 16;
 constexpr uint32_t CASE_BATCH = 1u << 20;  // pairs per device batch in run_case
 
@@ -119,10 +118,10 @@ struct collatz_ctx {
   uint32_t range64_bits = 48;
   uint32_t iter_cap = 1u << 16;
   // scratch for the synchronous calls
-  cz::DevBuf d_rec, d_counter, d_overflow, d_ovcount, d_pairs[2], d_segs, d_widen, d_widen2, d_wcount;
+  cz::DevBuf d_rec, d_counter, d_overflow, d_ovcount, d_pairs[2], d_segs, d_lists;
   cz::HostBuf h_rec, h_pairs;
   // one-shot range batches (collatz_verify_batch / collatz_verify_range)
-  cz::DevBuf d_recs, d_rcursor, d_first;  // d_first: per request, its first segment (threshold scouts)
+  cz::DevBuf d_recs, d_range;  // d_range: head, then records
   cz::HostBuf h_segs, h_recs;
   std::vector<cz::RangeSeg> range_segs;
   cz::DevBuf t_seeds, t_st, t_exc, t_status, t_idx[2], t_cnt;
@@ -156,20 +155,6 @@ int get_range_tables(collatz_ctx* c, uint32_t k, RangeTables** out, bool negativ
 cudaError_t range_kernel_launch(collatz_ctx* c, const RangeArgs& a, cudaStream_t s);
 int lower_range(collatz_ctx* c, const collatz_range& r, uint32_t req, const RangeTables& T,
                 std::vector<RangeSeg>& segs, unsigned long long& items);
-// The segment of segs[from..) with the most items (items: the end of the last one), from
-// which a request's scouts are taken; ~0u when there is none.
-inline uint32_t scout_segment(const std::vector<RangeSeg>& segs, size_t from, unsigned long long items) {
-  uint32_t best = ~0u;
-  unsigned long long most = 0;
-  for (size_t i = from; i < segs.size(); i++) {
-    const unsigned long long n = (i + 1 < segs.size() ? segs[i + 1].item_begin : items) - segs[i].item_begin;
-    if (n > most) {
-      most = n;
-      best = (uint32_t)i;
-    }
-  }
-  return best;
-}
 void rec_to_range_result(const ReqRec& r, collatz_range_result* out);
 // Applies cached autotuner choices to a new context (tune.cu).
 void tune_on_create(collatz_ctx* c);

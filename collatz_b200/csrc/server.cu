@@ -9,7 +9,7 @@
 //                    requests of one sieve exponent k (water-filling: requests
 //                    that need less than an equal share take what they need,
 //                    the rest of the slice budget goes to the larger ones),
-//                    followed by the 192- and 256-bit widening passes and a
+//                    followed by the candidate and wide-seed pass and a
 //                    copy of the request records; a prologue kernel zeroes the
 //                    slice's counters and the records of newly admitted
 //                    requests.  Two slices are kept in
@@ -90,7 +90,7 @@ struct Req {
 };
 
 struct Slice {
-  DevBuf d_segs, d_cursor, d_widen[2], d_wcount;
+  DevBuf d_segs, d_head, d_lists;
   HostBuf h_segs, h_recs;
   std::vector<Req*> finishing;
   cudaEvent_t t0 = nullptr, done = nullptr;
@@ -121,17 +121,12 @@ struct Batch {
 
 double since(Clock::time_point t0) { return std::chrono::duration<double>(Clock::now() - t0).count(); }
 
-// A slice's prologue: zeroes its item cursor and widen counters and the
+// A slice's prologue: zeroes its head (item cursor, list lengths) and the
 // records of the requests admitted since the previous slice (one launch in
 // place of a memset per request).
-__global__ void k_slice_prologue(unsigned long long* cursor, uint32_t* wcount, ReqRec* recs, const uint32_t* slots,
-                                 uint32_t nslots) {
+__global__ void k_slice_prologue(RangeHead* head, ReqRec* recs, const uint32_t* slots, uint32_t nslots) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t == 0) {
-    *cursor = 0;
-    wcount[0] = 0;
-    wcount[1] = 0;
-  }
+  if (t < sizeof(RangeHead) / 4) reinterpret_cast<uint32_t*>(head)[t] = 0u;
   constexpr uint32_t W = sizeof(ReqRec) / 8;  // 18 words of 8 bytes
   for (uint32_t i = t; i < nslots * W; i += gridDim.x * blockDim.x)
     reinterpret_cast<unsigned long long*>(recs + slots[i / W])[i % W] = 0ull;
@@ -444,15 +439,11 @@ int launch_slice(collatz_server* s, int si) {
   std::vector<RangeSeg> segs;
   unsigned long long slice_items = 0, budget = s->cfg.slice_items;
   uint32_t seed_bits = 0;
-  std::vector<uint32_t> scouts;  // the scouts' segment of each request that starts in this slice
   for (size_t i = 0; i < want.size(); i++) {
     const unsigned long long share = std::max<unsigned long long>(1, budget / (want.size() - i));
     const unsigned long long q = std::min(want[i].first, share);
     if (q) seed_bits = std::max(seed_bits, range_seed_bits(want[i].second->q.range));
-    const bool starts = want[i].second->cursor == 0;
-    const size_t before = segs.size();
     take_items(want[i].second, q, segs, slice_items);
-    if (starts && segs.size() > before) scouts.push_back(scout_segment(segs, before, slice_items));
     budget -= std::min(budget, q);
     if (want[i].second->cursor == want[i].second->items) S.finishing.push_back(want[i].second);
   }
@@ -460,17 +451,16 @@ int launch_slice(collatz_server* s, int si) {
   RangeTables* T = nullptr;
   int rc = get_range_tables(c, k, &T, neg);
   if (rc) return rc;
-  const size_t sb = sizeof(RangeSeg) * segs.size(), fb = sizeof(uint32_t) * scouts.size();
+  const size_t sb = sizeof(RangeSeg) * segs.size();
   const size_t zb = sizeof(uint32_t) * s->fresh_slots.size();
   const size_t rb = sizeof(ReqRec) * s->cfg.max_active;
-  // one upload: the segments, the scouts' segment indices, the records to zero
-  cudaError_t e = S.d_segs.ensure(sb + fb + zb);
-  if (!e) e = S.h_segs.ensure(sb + fb + zb);
+  // one upload: the segments, the records to zero
+  cudaError_t e = S.d_segs.ensure(sb + zb);
+  if (!e) e = S.h_segs.ensure(sb + zb);
   if (!e) e = S.h_recs.ensure(rb);
   if (e) return set_cuda_error(c, e, "server slice buffers");
   std::memcpy(S.h_segs.p, segs.data(), sb);
-  if (fb) std::memcpy(static_cast<char*>(S.h_segs.p) + sb, scouts.data(), fb);
-  if (zb) std::memcpy(static_cast<char*>(S.h_segs.p) + sb + fb, s->fresh_slots.data(), zb);
+  if (zb) std::memcpy(static_cast<char*>(S.h_segs.p) + sb, s->fresh_slots.data(), zb);
   const uint32_t nfresh = (uint32_t)s->fresh_slots.size();
   s->fresh_slots.clear();
   RangeArgs a;
@@ -478,38 +468,26 @@ int launch_slice(collatz_server* s, int si) {
   a.k = k;
   a.segs = S.d_segs.as<RangeSeg>();
   a.nsegs = (uint32_t)segs.size();
-  a.item_cursor = S.d_cursor.as<unsigned long long>();
   a.item_limit = slice_items;
   a.recs = s->d_recs.as<ReqRec>();
-  a.widen = S.d_widen[0].as<WidenEntry>();
-  a.widen_cap = WIDEN_CAP;
-  a.widen_count = S.d_wcount.as<uint32_t>();
+  a.head = S.d_head.as<RangeHead>();
+  a.lists = S.d_lists.as<RangeLists>();
   a.iter_cap = c->iter_cap;
   a.stats = nullptr;
   a.negative = neg ? 1u : 0u;
   a.seed_bits = seed_bits;
   cudaStream_t st = s->sa;
-  e = cudaMemcpyAsync(S.d_segs.p, S.h_segs.p, sb + fb + zb, cudaMemcpyHostToDevice, st);
+  e = cudaMemcpyAsync(S.d_segs.p, S.h_segs.p, sb + zb, cudaMemcpyHostToDevice, st);
   if (!e) {
     const uint32_t words = nfresh * (uint32_t)(sizeof(ReqRec) / 8);
     k_slice_prologue<<<std::max(1u, std::min(64u, (words + 255) / 256)), 256, 0, st>>>(
-        S.d_cursor.as<unsigned long long>(), S.d_wcount.as<uint32_t>(), s->d_recs.as<ReqRec>(),
-        reinterpret_cast<const uint32_t*>(static_cast<const char*>(S.d_segs.p) + sb + fb), nfresh);
+        S.d_head.as<RangeHead>(), s->d_recs.as<ReqRec>(),
+        reinterpret_cast<const uint32_t*>(static_cast<const char*>(S.d_segs.p) + sb), nfresh);
     e = cudaGetLastError();
   }
   if (!e) e = cudaEventRecord(S.t0, st);
-  // threshold scouts for the requests that start here (their records were zeroed by the prologue)
-  if (!e && fb)
-    e = launch_range_scout(a, reinterpret_cast<const uint32_t*>(static_cast<const char*>(S.d_segs.p) + sb),
-                           (uint32_t)scouts.size(), st);
   if (!e) e = range_kernel_launch(c, a, st);
-  if (!e)
-    e = launch_range_wide(S.d_widen[0].as<WidenEntry>(), S.d_wcount.as<uint32_t>(), WIDEN_CAP, 6, a.recs,
-                          S.d_widen[1].as<WidenEntry>(), WIDEN_CAP, S.d_wcount.as<uint32_t>() + 1, c->iter_cap, st,
-                          neg);
-  if (!e)
-    e = launch_range_wide(S.d_widen[1].as<WidenEntry>(), S.d_wcount.as<uint32_t>() + 1, WIDEN_CAP, 8, a.recs,
-                          nullptr, 0, nullptr, c->iter_cap, st, neg);
+  if (!e) e = launch_range_finish(a, st);
   if (!e && !S.finishing.empty()) e = cudaMemcpyAsync(S.h_recs.p, s->d_recs.p, rb, cudaMemcpyDeviceToHost, st);
   if (!e) e = cudaEventRecord(S.done, st);
   if (e) return set_cuda_error(c, e, "server slice launch");
@@ -851,10 +829,8 @@ void destroy(collatz_server* s) {
     if (s->sb) cudaStreamSynchronize(s->sb);
     for (Slice& S : s->slices) {
       S.d_segs.release();
-      S.d_cursor.release();
-      S.d_widen[0].release();
-      S.d_widen[1].release();
-      S.d_wcount.release();
+      S.d_head.release();
+      S.d_lists.release();
       S.h_segs.release();
       S.h_recs.release();
       if (S.t0) cudaEventDestroy(S.t0);
@@ -924,17 +900,15 @@ extern "C" int collatz_server_start(const collatz_config* cfg, const collatz_ser
   cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep);
   if ((e = s->d_recs.ensure(sizeof(ReqRec) * s->cfg.max_active))) return fail(e, "server records");
   for (Slice& S : s->slices) {
-    if ((e = S.d_cursor.ensure(sizeof(unsigned long long)))) return fail(e, "slice");
-    if ((e = S.d_widen[0].ensure(sizeof(WidenEntry) * WIDEN_CAP))) return fail(e, "slice");
-    if ((e = S.d_widen[1].ensure(sizeof(WidenEntry) * WIDEN_CAP))) return fail(e, "slice");
-    if ((e = S.d_wcount.ensure(2 * sizeof(uint32_t)))) return fail(e, "slice");
+    if ((e = S.d_head.ensure(sizeof(RangeHead)))) return fail(e, "slice");
+    if ((e = S.d_lists.ensure(sizeof(RangeLists)))) return fail(e, "slice");
     if ((e = cudaEventCreate(&S.t0))) return fail(e, "event");
     if ((e = cudaEventCreate(&S.done))) return fail(e, "event");
   }
   // Host and device staging is allocated here, once: growing a pinned or
   // device buffer later (cudaFreeHost / cudaFree synchronise the device,
   // large cudaMallocHost calls take milliseconds) would stall both workers.
-  // per request: its segments and one threshold-scout index
+  // per request: its segments
   const size_t seg_bytes = (sizeof(RangeSeg) * SEGS_PER_REQ + sizeof(uint32_t)) * s->cfg.max_active;
   for (Slice& S : s->slices) {
     if ((e = S.d_segs.ensure(seg_bytes))) return fail(e, "slice");
