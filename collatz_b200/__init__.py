@@ -72,8 +72,8 @@ class RangeResultC(C.Structure):
 
 REQ_RANGE, REQ_TRAJECTORY = 0, 1
 TUNE_RANGE, TUNE_CASES, TUNE_NO_CACHE = 0x1, 0x2, 0x4
-# collatz_set_variant modes: cases kernel, four-limb range kernel, 64-bit range
-# kernel, and the limb width (largest seed bit length run by the 64-bit kernel)
+# collatz_set_variant modes: cases kernel, range kernel with three and four words, range
+# kernel with two, and the width (largest seed bit length run with two words)
 MODE_CASES, MODE_RANGE, MODE_RANGE64, MODE_RANGE64_BITS = 0, 1, 2, 3
 RANGE64_BITS_DEFAULT = 48
 

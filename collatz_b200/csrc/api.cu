@@ -290,6 +290,7 @@ extern "C" int collatz_create(const collatz_config* cfg, collatz_ctx** out) {
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking);
   for (int i = 0; i < 4 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
   if (e == cudaSuccess) e = range_init(c->own_stream);
+  if (e == cudaSuccess) e = cases_win_init(c->own_stream);
   if (e == cudaSuccess) e = build_case_tables(&c->ct, cfg->maxbits, c->own_stream);
   if (e != cudaSuccess) {
     rc = set_cuda_error(c, e, "collatz_create");

@@ -326,4 +326,52 @@ static __device__ __noinline__ void rec_offer_e(ReqRec* r, const u32* E, const u
   rec_unlock(r);
 }
 
+// The same for all lanes of a warp together, one of them with mine (kind 0: st, 1: E of four
+// limbs), after the caller has raised the key to k or beyond.  DROP: an offer whose key is
+// beaten meanwhile is dropped without the lock (4736 warps that took it in turn for one
+// record's first offers needed 160 ms).  The loop has votes for its conditions: a spin by
+// one lane makes the compiler take the warp to be diverged at every later vote.
+template <bool DROP>
+__device__ __forceinline__ void rec_offer_vote(ReqRec* r, bool mine, u32 kind, ull k, u32 st, const u32* E, const u32* seed) {
+  if (!__any_sync(FULL, mine)) return;
+  bool got = false;
+#pragma unroll 1
+  for (u32 i = 0; i < LOCK_SPIN_LIMIT; i++) {
+    if (DROP) mine = mine && *(const volatile ull*)(kind ? &r->e_key : &r->st_key) <= k;
+    got = mine && atomicCAS(&r->lock, 0u, 1u) == 0u;
+    if (DROP ? !__any_sync(FULL, mine && !got) : __any_sync(FULL, got)) break;
+    __nanosleep(64);
+  }
+  if (got) {
+    __threadfence();
+    volatile ReqRec* v = r;
+    if (kind == 0) {
+      if (!(v->valid & 1u) || st > v->st || (st == v->st && seed_lt4(seed, v->st_seed))) {
+        v->st = st;
+        for (int j = 0; j < 4; j++) v->st_seed[j] = seed[j];
+        v->valid = v->valid | 1u;
+      }
+    } else {
+      bool lt = false, eq = true;  // E against the record's
+#pragma unroll 1
+      for (int j = 7; j >= 0; j--) {
+        const u32 x = j < 4 ? E[j & 3] : 0u, y = v->E[j];
+        lt = lt | (eq & (x < y));
+        eq = eq & (x == y);
+      }
+      if (!(v->valid & 2u) || (!lt && !eq) || (eq && seed_lt4(seed, v->E_seed))) {
+#pragma unroll 1
+        for (int j = 0; j < 8; j++) v->E[j] = j < 4 ? E[j & 3] : 0u;
+        for (int j = 0; j < 4; j++) v->E_seed[j] = seed[j];
+        v->valid = v->valid | 2u;
+      }
+    }
+    __threadfence();
+    atomicExch(&r->lock, 0u);
+  } else if (mine) {
+    atomicOr(&r->errors, ERR_LOCK);
+  }
+  __syncwarp();
+}
+
 }  // namespace cz

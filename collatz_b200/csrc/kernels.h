@@ -25,9 +25,13 @@ struct CasesArgs {
   unsigned long long* overflow_count;
   uint32_t iter_cap;       // checkpoints per seed before ERR_ITER_CAP
   uint32_t multi;          // line batch: base limb 3 = bigindex | line << 8, rec[line] per line
+  uint32_t four = 4, p5 = 1u << 5, p29 = 1u << 29;  // unknown to the compiler (cases_win.cu: additions and
+                                                    // shifts on the multiply-add pipe)
 };
 int cases_variants();
 cudaError_t launch_cases(const CasesArgs& a, int variant, uint32_t grid, cudaStream_t st);
+cudaError_t cases_win_init(cudaStream_t st);  // once per device, before the first launch; ends with st idle
+cudaError_t launch_cases_win(const CasesArgs& a, cudaStream_t st);  // N <= 52
 cudaError_t cases_occupancy(int variant, int* blocks_per_sm, bool multi = false);
 
 // ---------------- device Step 1 (step1_dev.cu) ----------------
@@ -141,10 +145,10 @@ struct RangeArgs {
   uint32_t seed_bits;             // bit length of the launch's largest seed (0: not known)
   uint32_t one = 1, mone = ~0u, eight = 8;  // 1, -1 and 8, unknown to the compiler (range.cu: window)
 };
-// Cases mode: seeds below 2^52 run the 64-bit body (measured on the range kernel's
-// run loop: 2^34 seeds at 2^51 took 5.20 ms with it and 5.21 ms without; at 2^52,
-// 5.29 ms and 5.21 ms).
-constexpr uint32_t RANGE_NARROW_MAX_BITS = 52;
+// Largest N that runs the kernel with run pairs from a table (cases_win.cu), whose values go to the
+// exact path from 2^71 on: at N = 48 a line of 304 724 seeds took 0.156 ms with it and 0.392
+// with four limbs, at N = 52 one of 3.75 M seeds 0.274 and 0.578.
+constexpr uint32_t CASES_WIN_MAX_BITS = 52;
 int range_variants();
 int range64_variants();
 // Hash of the variant table (part of the autotuner's cache key).

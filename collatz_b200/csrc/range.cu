@@ -268,44 +268,7 @@ __device__ __forceinline__ void offer(const RangeArgs& A, bool lead, const Range
     full = i >= CAND_CAP;
     if (!full) A.lists->cand[i] = c;
   }
-  if (!__any_sync(FULL, full)) return;
-  bool got = false;
-#pragma unroll 1
-  for (u32 i = 0; i < LOCK_SPIN_LIMIT; i++) {
-    got = full && atomicCAS(&r->lock, 0u, 1u) == 0u;
-    if (__any_sync(FULL, got)) break;
-    __nanosleep(64);
-  }
-  if (got) {
-    __threadfence();
-    volatile ReqRec* v = r;
-    if (c.kind == 0) {
-      if (!(v->valid & 1u) || c.st > v->st || (c.st == v->st && seed_lt4(c.seed, v->st_seed))) {
-        v->st = c.st;
-        for (int j = 0; j < 4; j++) v->st_seed[j] = c.seed[j];
-        v->valid = v->valid | 1u;
-      }
-    } else {
-      bool lt = false, eq = true;  // E against the record's
-#pragma unroll 1
-      for (int j = 7; j >= 0; j--) {
-        const u32 x = j < 4 ? c.E[j & 3] : 0u, y = v->E[j];
-        lt = lt | (eq & (x < y));
-        eq = eq & (x == y);
-      }
-      if (!(v->valid & 2u) || (!lt && !eq) || (eq && seed_lt4(c.seed, v->E_seed))) {
-#pragma unroll 1
-        for (int j = 0; j < 8; j++) v->E[j] = j < 4 ? c.E[j & 3] : 0u;
-        for (int j = 0; j < 4; j++) v->E_seed[j] = c.seed[j];
-        v->valid = v->valid | 2u;
-      }
-    }
-    __threadfence();
-    atomicExch(&r->lock, 0u);
-  } else if (full) {
-    atomicOr(&r->errors, ERR_LOCK);
-  }
-  __syncwarp();
+  rec_offer_vote<false>(r, full, c.kind, 0, c.st, c.E, c.seed);
 }
 
 // The exact path for the warp's queued seeds e (n limbs 0..2, request), one per

@@ -1,8 +1,8 @@
 // tune.cu -- autotuner for the kernel variants (collatz_autotune).
 //
-// The range kernel comes in variants of block shape (run pairs between
-// refills R, minimum resident blocks per SM), the cases kernel in variants of
-// checkpoints per pass and refill threshold.  The autotuner times every
+// The range kernel comes in variants of window length, refill thresholds and
+// warps per block, the cases kernel in variants of checkpoints per pass and
+// refill threshold, and a table-driven one.  The autotuner times every
 // variant of a mode on a fixed sample on this device, keeps the fastest for
 // the context, and records it in a small text cache keyed by the device, the
 // library's variant set and the workload parameter (range: sieve exponent k;
@@ -221,14 +221,14 @@ extern "C" int collatz_autotune(collatz_ctx* c, uint32_t flags, collatz_tune_res
     const int keep = c->range_variant, keep64 = c->range64_variant;
     const uint32_t keep_bits = c->range64_bits;
     const int nv = std::min(range_variants(), 8), nv64 = std::min(range64_variants(), 8);
-    c->range64_bits = 0;  // the four-limb kernel's variants
+    c->range64_bits = 0;  // the variants for three words
     for (int v = 0; v < nv && !rc; v++) {
       c->range_variant = v;
       rc = time_range(c, r, &res.range_ms[v]);
     }
     const int best = rc ? keep : (int)(std::min_element(res.range_ms, res.range_ms + nv) - res.range_ms);
     c->range_variant = best;
-    c->range64_bits = range64_max_seed_bits();  // the 64-bit kernel's variants
+    c->range64_bits = range64_max_seed_bits();  // the variants for two words
     for (int v = 0; v < nv64 && !rc; v++) {
       c->range64_variant = v;
       rc = time_range(c, r, &res.range64_ms[v]);
