@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 from dataclasses import dataclass, field
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -234,10 +235,21 @@ def _case_result(r: CaseResultC, ovbuf, cap) -> CaseResult:
                       r.max_stopping_time, _limbs(r.max_stopping_time_seed), r.errors, r.device_ms)
 
 
+# RangeResultC and Range as packed records: 1000 ctypes structures were filled and read field by
+# field in 6.0 ms, 20 times the launch they belong to.
+_RANGE_RESULT = struct.Struct("<QQQ32s16sQ16sIid")
+_RANGE = struct.Struct("<QQQII")
+assert _RANGE_RESULT.size == C.sizeof(RangeResultC) and _RANGE.size == C.sizeof(Range)
+
+
+def _range_results(out) -> list[RangeResult]:
+    n = int.from_bytes
+    return [RangeResult(a, b, c, n(e, "little"), n(es, "little"), t, n(ts, "little"), err, st, ms)
+            for a, b, c, e, es, t, ts, err, st, ms in _RANGE_RESULT.iter_unpack(out)]
+
+
 def _range_result(r: RangeResultC) -> RangeResult:
-    return RangeResult(r.seeds_checked, r.failures, r.widened, _limbs(r.max_excursion),
-                       _limbs(r.max_excursion_seed), r.max_stopping_time,
-                       _limbs(r.max_stopping_time_seed), r.errors, r.status, r.device_ms)
+    return _range_results(r)[0]
 
 
 def make_case(base, sigfig, threepower, number, doubleeven, numevens) -> Case:
@@ -256,6 +268,19 @@ def make_range(offset: int, size: int, k: int = 0, mod9: bool = True, negative: 
     r.size, r.k = size, k
     r.flags = (0 if mod9 else RANGE_NO_MOD9) | (RANGE_NEGATIVE if negative else 0)
     return r
+
+
+def _pack_range(offset, size, k=0, mod9=True, negative=False) -> bytes:
+    if type(offset) is not int or type(size) is not int or type(k) is not int:
+        return bytes(make_range(offset, size, k, mod9, negative))
+    m = 2**64 - 1
+    return _RANGE.pack(offset & m, offset >> 64 & m, size & m, k & 0xFFFFFFFF,
+                       (0 if mod9 else RANGE_NO_MOD9) | (RANGE_NEGATIVE if negative else 0))
+
+
+def _ranges(reqs) -> "C.Array":
+    """[(offset, size[, k[, mod9[, negative]]])] -> Range array, as make_range of each."""
+    return (Range * len(reqs)).from_buffer_copy(b"".join([_pack_range(*q) for q in reqs]))
 
 
 def pack_pairs(pairs) -> "C.Array":
@@ -528,14 +553,12 @@ class Verifier:
     def verify_batch(self, reqs, check: bool = True) -> list[RangeResult]:
         """reqs: [(offset, size)] or [(offset, size, k, mod9)]."""
         n = len(reqs)
-        arr = (Range * n)()
-        for i, q in enumerate(reqs):
-            arr[i] = make_range(*q)
+        arr = _ranges(reqs)
         out = (RangeResultC * n)()
         rc = lib().collatz_verify_batch(self._h, arr, n, out)
         if check:
             self._check(rc, "verify_batch")
-        return [_range_result(out[i]) for i in range(n)]
+        return _range_results(out)
 
     def plan(self, reqs) -> "Plan":
         return Plan(self, reqs)
@@ -575,9 +598,7 @@ class Plan:
     def __init__(self, v: Verifier, reqs):
         self.v = v
         self.n = len(reqs)
-        arr = (Range * self.n)()
-        for i, q in enumerate(reqs):
-            arr[i] = make_range(*q)
+        arr = _ranges(reqs)
         h = C.c_void_p()
         v._check(lib().collatz_plan_create(v.handle, arr, self.n, C.byref(h)), "plan_create")
         self._h = h
@@ -590,7 +611,7 @@ class Plan:
         rc = lib().collatz_plan_results(self._h, out)
         if check:
             self.v._check(rc, "plan_results")
-        return [_range_result(out[i]) for i in range(self.n)]
+        return _range_results(out)
 
     def close(self):
         if getattr(self, "_h", None):
