@@ -427,7 +427,8 @@ __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_const
         t = (u64)a * r1.z + r0.w + (t >> 32);
         w1 = (u32)t;
         t = (u64)a * r1.w + r1.x + (t >> 32);
-        w2 = ((t >> 32) | r2.w) ? FULL : (u32)t;  // (2^80 and beyond: to the exact path)
+        // (0, which would read as none, and 2^80 and beyond: to the exact path)
+        w2 = ((t >> 32) | r2.w) != 0 || (w0 | w1 | (u32)t) == 0 ? FULL : (u32)t;
         nlim = r2.x;
         npair = r2.y;
         na10 = a;

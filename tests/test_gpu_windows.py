@@ -43,6 +43,7 @@ def test_pair_look_ups_match_oracle(verifier, oracle_tables, n, bits):
     mask = (1 << (n - 10)) - 1
     pairs = [((0x9E3779B97F4A7C15 * (i + 1)) & mask, (1 << bits) - 12345 + 4097 * i) for i in range(8)]
     pairs += pairs[:1] * 40  # more pairs than a warp's slots
+    pairs += [(pairs[1][0], 0)]  # a value of 0 for a = 0
     r = v.launchkernel(3, pairs)
     o = T.pairs_result(3, pairs)
     assert (r.hash, r.seeds_checked, r.errors) == (o.hash, o.seeds, 0)
