@@ -57,12 +57,13 @@ WORK_MODEL = {"block": {"words": 2, "windows": 1.81}, "frontier": {"words": 3, "
 #   block:    k_range on two-word values, 2^34 launch at 2^40, k = 24 (dram bytes per
 #             launch do not grow with the block: the 4.6 MB survivor table is read
 #             from DRAM once and from L2 after that);
-#   frontier: k_range on three-word values, 2^36 launch at 2^60, k = 34.
+#   frontier: k_range on three-word values, at 2^60, k = 34: the pipes of a 2^36 launch, the dram
+#             bytes of a 2^40 launch (the 2.43 GB table about twice, however many blocks).
 NCU_CAPTURES = {
-    "block": {"src": "", "dram_bytes": 0, "per": "launch",
-              "issue_slots_busy": 0, "alu_pipe_busy": 0, "kernel": "k_range (two words)"},
-    "frontier": {"src": "", "dram_bytes": 0, "per": "launch",
-                 "issue_slots_busy": 0, "alu_pipe_busy": 0, "kernel": "k_range (three words)"},
+    "block": {"src": "4b78aec381e29935", "dram_bytes": 4.674560e6 + 0.002048e6, "per": "launch",
+              "issue_slots_busy": 0.7529, "alu_pipe_busy": 0.6507, "kernel": "k_range (two words)"},
+    "frontier": {"src": "4b78aec381e29935", "dram_bytes": 5.180748e9 + 1.15155712e8, "per": "launch",
+                 "issue_slots_busy": 0.7963, "alu_pipe_busy": 0.7030, "kernel": "k_range (three words)"},
 }
 SHARED_KERNEL_SOURCES = ("common.cuh", "kernels.h", "tables.h", "tables.cu")
 KERNEL_SOURCES = {"block": ("range.cu",) + SHARED_KERNEL_SOURCES,
@@ -816,15 +817,15 @@ def main():
                         "max_excursion": str(res.max_excursion),
                         "max_excursion_seed": str(res.max_excursion_seed), "errors": res.errors},
             "roofline": roof,
-            # request (32 B) + its work list: an aligned range of many blocks lowers to 55
-            # 64-byte segments (5 kept mod-9 classes of the first and last block, 9 x 5 for the
-            # blocks between), and the request's 4-byte first-segment index (threshold scouts)
-            "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 32 + 64 * 55 + 4,
+            # request (32 B) + its work list: an aligned range of many blocks lowers to 19
+            # 64-byte segments (5 kept mod-9 classes of the first and last block, 9 for the
+            # blocks between)
+            "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 32 + 64 * 19,
                     "d2h_bytes_per_step": 144,
                     "call": "collatz_verify_range (lower + upload work list + launches + result copy)"},
             "clocks": clocks,
-            # per step: k_range_scout, k_range and the two widening passes
-            "gpu_launches": 4 * args.steps,
+            # per step: k_range and k_range_finish
+            "gpu_launches": 2 * args.steps,
             "wall_s_timed": wall,
         }
         nthreads = os.cpu_count() or 1

@@ -361,13 +361,13 @@ int collatz_server_stop(collatz_server *s);
 
 /* Kernel choices for the autotuner (no counterpart in the reference).
  *   COLLATZ_MODE_CASES, COLLATZ_MODE_RANGE: variant (block shape, body) of
- *     the cases kernel and of the four-limb range kernel;
- *   COLLATZ_MODE_RANGE64: variant of the 64-bit range kernel (jump-table
- *     window of 10 or 11 steps, run pairs at expansion, warp votes per step,
- *     queue-pop threshold, blocks per SM);
- *   COLLATZ_MODE_RANGE64_BITS: the limb width -- launches whose seeds all have
- *     at most this many bits (0..52) run the 64-bit kernel, the others the
- *     four-limb kernel (0: always four limbs).
+ *     the cases kernel and of the range kernel for values of three and four
+ *     32-bit words;
+ *   COLLATZ_MODE_RANGE64: variant of the range kernel for values of two words
+ *     (window length, refill thresholds, warps per block);
+ *   COLLATZ_MODE_RANGE64_BITS: the width -- launches whose seeds all have at
+ *     most this many bits (0..52; those above 48 count as 48) keep values in
+ *     two words, the others in three or four (0: never two).
  * collatz_variant_count gives the number of choices (0..count-1). */
 #define COLLATZ_MODE_CASES 0
 #define COLLATZ_MODE_RANGE 1
@@ -378,13 +378,11 @@ int collatz_set_variant(collatz_ctx *ctx, int mode, int variant);
 
 /* Autotuner (no counterpart in the reference).  Times every variant of the
  * selected modes on a fixed sample on this device and keeps the fastest:
- *   range: the four-limb kernel's variants and the 64-bit kernel's variants
- *     (window length j of the jump table, windows and run pairs per seed at
- *     expansion, in-loop table steps) on 2^34 seeds at 2^40 with the
- *     context's k, then the limb width: the two best variants timed on the
+ *   range: the range kernel's variants with the width at 0 and at its maximum
+ *     (window length, refill thresholds, warps per block) on 2^34 seeds at 2^40
+ *     with the context's k, then the width: the two best variants timed on the
  *     2^32 largest seeds of 44 bits and of 48 bits; range64_bits is the
- *     largest of 48, 44 at which the 64-bit kernel is faster, else 0 (four
- *     limbs throughout);
+ *     largest of 48, 44 at which two words are faster, else 0;
  *   cases: about 2^20 Step-1 pairs of the root case "3 2 2 9 1 0" for the
  *     context's N.
  * The choices go into a text cache (COLLATZ_TUNE_CACHE, else
@@ -396,10 +394,10 @@ int collatz_set_variant(collatz_ctx *ctx, int mode, int variant);
 typedef struct {
   int32_t range_variant, cases_variant; /* chosen (or kept when not tuned) */
   float range_ms[8], cases_ms[8];       /* device ms per variant on the sample; -1 = not timed */
-  int32_t range64_variant;              /* 64-bit range kernel: chosen variant */
-  uint32_t range64_bits;                /* chosen limb width (COLLATZ_MODE_RANGE64_BITS) */
-  float range64_ms[8];                  /* device ms per 64-bit variant on the sample; -1 = not timed */
-  float width_ms[4];                    /* 44-bit seeds: four limbs, 64 bits; 48-bit seeds: four limbs, 64 bits */
+  int32_t range64_variant;              /* two words: chosen variant */
+  uint32_t range64_bits;                /* chosen width (COLLATZ_MODE_RANGE64_BITS) */
+  float range64_ms[8];                  /* device ms per two-word variant on the sample; -1 = not timed */
+  float width_ms[4];                    /* 44-bit seeds: width 0, two words; 48-bit seeds: the same */
 } collatz_tune_result;
 #define COLLATZ_TUNE_RANGE 0x1u
 #define COLLATZ_TUNE_CASES 0x2u
