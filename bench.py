@@ -60,10 +60,10 @@ WORK_MODEL = {"block": {"words": 2, "windows": 1.81}, "frontier": {"words": 3, "
 #   frontier: k_range on three-word values, at 2^60, k = 34: the pipes of a 2^36 launch, the dram
 #             bytes of a 2^40 launch (the 2.43 GB table about twice, however many blocks).
 NCU_CAPTURES = {
-    "block": {"src": "4b78aec381e29935", "dram_bytes": 4.674560e6 + 0.002048e6, "per": "launch",
-              "issue_slots_busy": 0.7529, "alu_pipe_busy": 0.6507, "kernel": "k_range (two words)"},
-    "frontier": {"src": "4b78aec381e29935", "dram_bytes": 5.180748e9 + 1.15155712e8, "per": "launch",
-                 "issue_slots_busy": 0.7963, "alu_pipe_busy": 0.7030, "kernel": "k_range (three words)"},
+    "block": {"src": "f2c27558ed8bb969", "dram_bytes": 4.679936e6 + 0.000768e6, "per": "launch",
+              "issue_slots_busy": 0.7515, "alu_pipe_busy": 0.6494, "kernel": "k_range (two words)"},
+    "frontier": {"src": "f2c27558ed8bb969", "dram_bytes": 5.180748e9 + 1.15155712e8, "per": "launch",
+                 "issue_slots_busy": 0.7961, "alu_pipe_busy": 0.7025, "kernel": "k_range (three words)"},
 }
 SHARED_KERNEL_SOURCES = ("common.cuh", "kernels.h", "tables.h", "tables.cu")
 KERNEL_SOURCES = {"block": ("range.cu",) + SHARED_KERNEL_SOURCES,

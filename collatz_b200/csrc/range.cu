@@ -1194,7 +1194,14 @@ static cudaError_t launch_t(const RangeArgs& a, int variant, u32 grid, cudaStrea
   return cudaGetLastError();
 }
 
+// Variant 0 with fewer than 512 rows to a warp runs with 24 warps per block: such launches spend
+// much of their time opening runs and on the exact path's last seeds, and fewer warps open
+// fewer.  2^28 seeds at 2^40: 115 us with 32 warps, 103 with 24; 2^30: 163 and 152; 2^32: 285
+// and 271; 2^30 at 2^60: 178 and 165.  Long launches need the 32 (2^36: 2.36 and 2.57 ms).
+constexpr int SMALL_VARIANT = 7;
+
 cudaError_t launch_range(const RangeArgs& a, int words, int variant, u32 sm_count, cudaStream_t st) {
+  if (variant == 0 && a.item_limit < 512ull * 32 * sm_count) variant = SMALL_VARIANT;
   const u32 grid = (u32)std::max<unsigned long long>(1, std::min<unsigned long long>(sm_count, a.item_limit));
   switch (words) {
     case 2: return launch_t<2>(a, variant, grid, st);
