@@ -11,7 +11,7 @@
 //
 // Stopping times and excursions are only bounded on the way.  A seed whose value
 // reaches 1/256 of the line's maximum excursion (a look-up's odd runs raise it by less than
-// 1.5^12 = 130) or 2^71, or whose look-ups could hold as many steps as the line's longest
+// 1.5^12 = 130) or a bound below 2^71 (case_limits.h), or whose look-ups could hold as many steps as the line's longest
 // stopping time, is queued and run again from its start, pair by pair with four limbs:
 // overflow reports, exact maxima, its hash (exact_batch).  No other seed can change a
 // maximum, report an overflow or reach the checkpoint cap.
@@ -19,6 +19,7 @@
 
 #include <algorithm>
 
+#include "case_limits.h"
 #include "common.cuh"
 #include "kernels.h"
 #include "tables.h"
@@ -32,7 +33,6 @@ constexpr u32 WCLAIM = 16;     // pairs per claim while many remain
 constexpr int WGROUP = 4;      // look-ups between two looks at the lanes
 constexpr int WREFILL = 20;    // lanes without a next seed that call for a refill
 constexpr u32 CP_BITS = 13;    // low bits of a look-up
-constexpr int CP_STEPS = 12;   // most steps of a look-up
 constexpr int IDLE_CNT = 1 << 30;
 
 // Entries, [0] before a checkpoint's first pair, [1] before its second: t << 12 | (1: a first pair was
@@ -97,17 +97,6 @@ __device__ __forceinline__ u32 lds32(u32 at) {
   u32 v;
   asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at));
   return v;
-}
-
-// A line's limits from its keys: the least value that goes to the exact path, in units of 2^48 (below
-// 2^24; 0: every value), and above it the look-ups that a seed may take (at most 200).
-__device__ __forceinline__ u32 line_limits(ull sk, ull ek, u32 mbi, u32 iter_cap) {
-  const int bl = (int)(ek >> 54);
-  const u32 hi = bl > 79 ? 1u << 23 : bl < 57 ? 0u : (u32)((ek & ((1ull << 54) - 1)) >> (110 - bl));
-  const u32 st = (u32)min(sk, 1ull << 24);
-  int k = st > mbi ? (int)((st - 1u - mbi) / (u32)CP_STEPS) : -1;
-  k = min(k, (int)min(iter_cap, 201u) - 1);  // (look-ups are at least the checkpoints)
-  return k < 0 ? 0u : hi | ((u32)k << 24);
 }
 
 // The queued seeds of all lanes with have, from their starts to their last checkpoints:
@@ -241,16 +230,17 @@ __device__ __forceinline__ void exact_batch(const CasesArgs& A, uint2 e, bool ha
 }
 
 // Lane state: v (0: idle; a fixed point of the look-ups that leaves the hash alone), n, the seed's
-// hash so far, the largest v / 2^48 and its limit, the look-ups left, the address of the
+// hash so far, the largest v in the limit's units and that limit, the look-ups left, the address of the
 // table for its next look-up; and the lane's next seed, so that a refill serves most lanes.
 // Bound by issue (77 % busy, the ALU 73 %): 19.7 warp instructions per seed against 49.7 with
 // the runs counted in 64-bit pairs; a seed takes about six look-ups, so that half the
 // instructions hand seeds to lanes.  555 M seeds of one line: 21.7 -> 9.6 ms, 2048 lines:
 // 14.2 -> 6.5 ms.  Groups of 3 look-ups 9.9 ms, of 2 10.6; a refill at 26 lanes 9.7; without
 // the next seed in the lane 10.1; 24 warps with 80 registers 10.1.
-template <bool MULTI>
+template <bool MULTI, u32 UNIT>
 __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_constant__ CasesArgs A) {
   CwShared& S = *reinterpret_cast<CwShared*>(cw_smem);
+  const u32 unit = UNIT ? UNIT : A.unit;
   for (u32 i = threadIdx.x; i < (2u << CP_BITS); i += WWARPS * 32) (&S.tab[0][0])[i] = (&g_cp[0][0])[i];
   if (threadIdx.x < 16) {
     u32 p = 1;
@@ -311,7 +301,7 @@ __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_const
       __syncwarp();
       {  // the lines' maxima may have risen
         const ReqRec* r = A.rec + W.ring[lane][2].z;
-        W.ring[lane][2].x = line_limits(*(volatile const ull*)&r->st_key, *(volatile const ull*)&r->e_key, mbi, A.iter_cap);
+        W.ring[lane][2].x = line_limits(*(volatile const ull*)&r->st_key, *(volatile const ull*)&r->e_key, mbi, A.iter_cap, unit);
       }
       __syncwarp();
       v0 = keep[0];
@@ -365,7 +355,7 @@ __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_const
         const u32 m0 = __shfl_sync(FULL, pw, 4), n3 = __shfl_sync(FULL, pw, 7);
         const u32 pline = MULTI ? (b3 >> 8) : 0u;
         const ReqRec* prec = A.rec + pline;
-        const u32 lim = line_limits(*(volatile const ull*)&prec->st_key, *(volatile const ull*)&prec->e_key, mbi, A.iter_cap);
+        const u32 lim = line_limits(*(volatile const ull*)&prec->st_key, *(volatile const ull*)&prec->e_key, mbi, A.iter_cap, unit);
         const u32 bi = (A.bigindex >= 0) ? (u32)A.bigindex : (MULTI ? (b3 & 0xFFu) : b3);
         u32 f = A.tpo + bi;
         if (f >= POW3_COUNT) f = POW3_COUNT - 1;
@@ -461,7 +451,7 @@ __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_const
         v1 = (u32)w;
         v2 = (v2 >> (e & 31u)) * m + (u32)(w >> 32);
         asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(hb) : "r"(e & CP_HALF), "r"(A.p5), "r"(tab));
-        mx = max(mx, __funnelshift_r(v1, v2, 16));
+        mx = max(mx, __funnelshift_r(v1, v2, unit));
         // at a checkpoint: the hash; below n: idle
         asm("{\n\t.reg .pred p, q;\n\t.reg .u32 t;\n\t.reg .u64 v, n;\n\t"
             "and.b32 t, %3, 0x200;\n\t"
@@ -490,7 +480,7 @@ __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_const
           v2 >>= b;
           add_carry3(v1, v2, v3, (v0 == 0) & (b != 0));
           cnt -= 4;  // (at most 39 steps)
-          mx = max(mx, __funnelshift_r(v1, v2, 16));
+          mx = max(mx, __funnelshift_r(v1, v2, unit));
           if (hb != tab) {
             hs ^= v0;
             if (v2 == 0 && (((u64)v1 << 32) | v0) < (((u64)n1 << 32) | n0)) v0 = v1 = 0;
@@ -526,7 +516,7 @@ __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_const
         const bool none = (w0 | w1 | w2) == 0;
         pair = none ? FULL : npair;
         a10 = na10;
-        mx = v2 >> 16 ? FULL : __funnelshift_r(v1, v2, 16);
+        mx = v2 >> unit ? FULL : __funnelshift_r(v1, v2, unit);
         hi = nlim & 0xFFFFFFu;
         cnt = none ? IDLE_CNT : (int)(nlim >> 24);
         w0 = w1 = w2 = 0;
@@ -548,9 +538,14 @@ __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_const
   if (lane == 0 && warp_seeds) atomicAdd(&A.rec[MULTI ? wline : 0].seeds, (ull)warp_seeds);
 }
 
+// Lines of N >= 45 have the largest unit: it is compiled in there (2048 lines of N = 45 took 7.73 ms with
+// the unit from the arguments and 7.61 so).
+constexpr u32 MAX_UNIT = 16;
+
 cudaError_t cases_win_init(cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(k_cases_win<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CwShared));
-  if (!e) e = cudaFuncSetAttribute(k_cases_win<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CwShared));
+  cudaError_t e = cudaSuccess;
+  for (auto k : {k_cases_win<false, 0>, k_cases_win<true, 0>, k_cases_win<false, MAX_UNIT>, k_cases_win<true, MAX_UNIT>})
+    if (!e) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CwShared));
   if (e) return e;
   k_cp_tables<<<(1u << CP_BITS) / 256, 256, 0, st>>>();
   e = cudaGetLastError();
@@ -563,8 +558,11 @@ cudaError_t launch_cases_win(const CasesArgs& a, cudaStream_t st) {
   if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e) return e;
   const u32 grid = std::min((u32)sms, std::max(1u, a.npairs));
-  if (a.multi) k_cases_win<true><<<grid, WWARPS * 32, sizeof(CwShared), st>>>(a);
-  else k_cases_win<false><<<grid, WWARPS * 32, sizeof(CwShared), st>>>(a);
+  CasesArgs b = a;
+  b.unit = line_unit(a.mbi + 10u);
+  const auto k = b.unit == MAX_UNIT ? (b.multi ? k_cases_win<true, MAX_UNIT> : k_cases_win<false, MAX_UNIT>)
+                                    : (b.multi ? k_cases_win<true, 0> : k_cases_win<false, 0>);
+  k<<<grid, WWARPS * 32, sizeof(CwShared), st>>>(b);
   return cudaGetLastError();
 }
 

@@ -25,6 +25,7 @@ struct CasesArgs {
   unsigned long long* overflow_count;
   uint32_t iter_cap;       // checkpoints per seed before ERR_ITER_CAP
   uint32_t multi;          // line batch: base limb 3 = bigindex | line << 8, rec[line] per line
+  uint32_t unit = 0;       // of the table-driven kernel's limits (case_limits.h), set by its launcher
   uint32_t four = 4, p5 = 1u << 5, p29 = 1u << 29;  // unknown to the compiler (cases_win.cu: additions and
                                                     // shifts on the multiply-add pipe)
 };
