@@ -21,6 +21,7 @@
 
 #include "case_limits.h"
 #include "common.cuh"
+#include "fill_once.h"
 #include "kernels.h"
 #include "tables.h"
 
@@ -39,6 +40,7 @@ constexpr int IDLE_CNT = 1 << 30;
 // taken) << 10 | (1: at a checkpoint) << 9 | f << 5 | s; s = 0: no pair ends.
 constexpr u32 CP_HALF = 1u << 10, CP_DONE = 1u << 9, CP_F = 0xFu << 5;
 __device__ u32 g_cp[2][1u << CP_BITS];
+__device__ u32 g_cp_ready;  // 1: the tables are filled
 
 __global__ void k_cp_tables() {
   const u32 m = blockIdx.x * blockDim.x + threadIdx.x;  // low bits of v
@@ -547,9 +549,13 @@ cudaError_t cases_win_init(cudaStream_t st) {
   for (auto k : {k_cases_win<false, 0>, k_cases_win<true, 0>, k_cases_win<false, MAX_UNIT>, k_cases_win<true, MAX_UNIT>})
     if (!e) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CwShared));
   if (e) return e;
-  k_cp_tables<<<(1u << CP_BITS) / 256, 256, 0, st>>>();
-  e = cudaGetLastError();
-  return e ? e : cudaStreamSynchronize(st);
+  return fill_once([&](bool* done) { return table_ready(g_cp_ready, done, st); },
+                   [&] {
+                     k_cp_tables<<<(1u << CP_BITS) / 256, 256, 0, st>>>();
+                     const cudaError_t l = cudaGetLastError();
+                     return l ? l : cudaStreamSynchronize(st);
+                   },
+                   [&] { return mark_table(g_cp_ready, st); });
 }
 
 cudaError_t launch_cases_win(const CasesArgs& a, cudaStream_t st) {

@@ -374,4 +374,18 @@ __device__ __forceinline__ void rec_offer_vote(ReqRec* r, bool mine, u32 kind, u
   __syncwarp();
 }
 
+// The mark that a table in device memory is filled: reading and setting it, ending with st idle.
+static inline cudaError_t table_ready(const u32& mark, bool* ready, cudaStream_t st) {
+  u32 v = 0;
+  cudaError_t e = cudaMemcpyFromSymbolAsync(&v, mark, sizeof v, 0, cudaMemcpyDeviceToHost, st);
+  if (!e) e = cudaStreamSynchronize(st);
+  *ready = v != 0;
+  return e;
+}
+static inline cudaError_t mark_table(u32& mark, cudaStream_t st) {
+  const u32 v = 1;
+  const cudaError_t e = cudaMemcpyToSymbolAsync(mark, &v, sizeof v, 0, cudaMemcpyHostToDevice, st);
+  return e ? e : cudaStreamSynchronize(st);
+}
+
 }  // namespace cz

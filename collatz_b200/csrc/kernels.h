@@ -31,7 +31,8 @@ struct CasesArgs {
 };
 int cases_variants();
 cudaError_t launch_cases(const CasesArgs& a, int variant, uint32_t grid, cudaStream_t st);
-cudaError_t cases_win_init(cudaStream_t st);  // once per device, before the first launch; ends with st idle
+// For every context, before its first launch; the tables are filled by a device's first.  Ends with st idle.
+cudaError_t cases_win_init(cudaStream_t st);
 cudaError_t launch_cases_win(const CasesArgs& a, cudaStream_t st);  // N <= 52
 cudaError_t cases_occupancy(int variant, int* blocks_per_sm, bool multi = false);
 
@@ -156,7 +157,7 @@ int range64_variants();
 uint32_t range_variant_rev();
 // Launches whose seeds have at most this many bits may run on two-word values.
 uint32_t range64_max_seed_bits();
-cudaError_t range_init(cudaStream_t st);  // once per device, before the first launch; ends with st idle
+cudaError_t range_init(cudaStream_t st);  // as cases_win_init
 // The range kernel with values of 2, 3 or 4 words (a seed that outgrows them
 // takes the kernel's exact path, so any width gives the same results).
 cudaError_t launch_range(const RangeArgs& a, int words, int variant, uint32_t sm_count, cudaStream_t st);

@@ -49,6 +49,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "fill_once.h"
 #include "kernels.h"
 #include "tables.h"
 
@@ -100,6 +101,7 @@ constexpr u32 WIN_M = 0x780u;
 __device__ u32 g_win[2][2][MAX_JW - MIN_JW + 1][1u << MAX_JW];
 // The largest D_i of the window, in units of 16, rounded up (for the screen).
 __device__ uint8_t g_peak[2][MAX_JW - MIN_JW + 1][1u << MAX_JW];
+__device__ u32 g_win_ready;  // 1: the tables above are filled
 // P = U << 16 | D (k_range) changes by P_ODD with each odd step of a window and by P_STEP with each step.
 constexpr u32 P_ODD = (u32)(-DA * 65535), P_STEP = (u32)(DB * 65535);
 
@@ -1223,15 +1225,20 @@ static cudaError_t init_t() {
   return e;
 }
 
-// Opts every range kernel into its dynamic shared memory and fills the window tables.
+// Opts every range kernel into its dynamic shared memory and fills the window tables if the device
+// has not got them yet.
 cudaError_t range_init(cudaStream_t st) {
   cudaError_t e = init_t<2>();
   if (e == cudaSuccess) e = init_t<3>();
   if (e == cudaSuccess) e = init_t<4>();
   if (e != cudaSuccess) return e;
-  k_win_tables<<<(1u << MAX_JW) / 256, 256, 0, st>>>();
-  e = cudaGetLastError();
-  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+  return fill_once([&](bool* done) { return table_ready(g_win_ready, done, st); },
+                   [&] {
+                     k_win_tables<<<(1u << MAX_JW) / 256, 256, 0, st>>>();
+                     const cudaError_t l = cudaGetLastError();
+                     return l ? l : cudaStreamSynchronize(st);
+                   },
+                   [&] { return mark_table(g_win_ready, st); });
 }
 
 cudaError_t launch_range_finish(const RangeArgs& a, cudaStream_t st) {
