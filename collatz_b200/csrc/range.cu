@@ -928,8 +928,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
             if (cu.mod9 && !(((A.negative ? KEEP9N : KEEP9) >> (u32)(n % 9u)) & 1u))
               cnt = (A.negative && n == 5) ? 1 : 0;
             te = ti + 4 * cnt + 4;
-            if (n < 2 && cnt) {
+            if (n < 2 && cnt) {  // 0 and 1 are not run: the entry begins with its second seed
               ti += 4;
+              g = gap_at(ti);
               cnt--;
             }
           }
