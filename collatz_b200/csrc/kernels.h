@@ -145,6 +145,7 @@ struct RangeArgs {
   uint32_t negative;              // 1: the negative-integer variant (a table built for it)
   unsigned long long* stats;      // diagnostics: [0] runs of rows, [1] seeds on the exact path; may be null
   uint32_t seed_bits;             // bit length of the launch's largest seed (0: not known)
+  uint32_t rl = 0, rs = 0;        // the variant's thresholds (range_variants.h), set by launch_range
   uint32_t one = 1, mone = ~0u, eight = 8;  // 1, -1 and 8, unknown to the compiler (range.cu: window)
 };
 // Largest N that runs the kernel with run pairs from a table (cases_win.cu), whose values go to the

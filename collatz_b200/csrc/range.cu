@@ -51,6 +51,7 @@
 #include "common.cuh"
 #include "fill_once.h"
 #include "kernels.h"
+#include "range_variants.h"
 #include "tables.h"
 
 namespace cz {
@@ -724,10 +725,9 @@ __device__ __forceinline__ ulonglong2 scout(const SH& S, const RangeArgs& A, u32
 }
 
 // The kernel.  It makes no function calls: with one, the compiler takes the warp to be
-// possibly diverged at every vote and spends three instructions on each.  L: words of a value; JW: window length; RL, RS: a warp gives its idle lanes new
-// entries once this many are idle, in runs of at least 64 rows and in shorter ones;
-// WARPS per block, one block per SM.
-template <int L, int JW, int RL, int RS, int WARPS>
+// possibly diverged at every vote and spends three instructions on each.  L: words of a value; JW:
+// window length; WARPS per block, one block per SM.
+template <int L, int JW, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__ RangeArgs A) {
   typedef RangeShared<JW, WARPS> Shared;
   Shared& S = *reinterpret_cast<Shared*>(range_smem);
@@ -977,7 +977,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
           ring++;
           next = 0;
           ents = __reduce_max_sync(FULL, nx.ents);  // (a reduction and a vote, so that they are known to be uniform)
-          thr = __any_sync(FULL, nx.rows >= 64) ? RL : RS;
+          thr = (int)(__any_sync(FULL, nx.rows >= 64) ? A.rl : A.rs);
           ulonglong2 keys = W.keys;
           if (__any_sync(FULL, keys.x == 0 && nx.ents != 0 && nx.small == 0)) {
             const bool have = lane < nx.ents;
@@ -1161,55 +1161,45 @@ __global__ void __launch_bounds__(128) k_range_finish(const __grid_constant__ Ra
 // Launchers.
 // ------------------------------------------------------------------
 
-// (window length JW, idle lanes that call for new entries in long and in short runs, warps per block)
-#define CZ_RANGE_VARIANTS(X)                                                                       \
-  X(0, 13, 4, 10, 32) X(1, 13, 4, 8, 32) X(2, 13, 4, 14, 32) X(3, 13, 2, 12, 32) X(4, 13, 6, 10, 32) X(5, 12, 4, 10, 32) \
-  X(6, 13, 4, 10, 28) X(7, 13, 4, 10, 24)
-
-int range_variants() { return 8; }
-int range64_variants() { return 8; }
+int range_variants() { return RANGE_VARIANTS; }
+int range64_variants() { return RANGE_VARIANTS; }
 uint32_t range64_max_seed_bits() { return 48; }
 
 // FNV-1a of the variant table's parameters: part of the autotuner's cache key, so that a
 // choice cached for another table is not applied to this one.
 uint32_t range_variant_rev() {
-  static const int p[] = {
-#define X(id, jw, rl, rs, wp) id, jw, rl, rs, wp,
-      CZ_RANGE_VARIANTS(X)
-#undef X
-  };
-  uint32_t h = 2166136261u;
-  for (int x : p) h = (h ^ (uint32_t)x) * 16777619u;
+  u32 h = 2166136261u;
+  for (const RangeVariant& v : RANGE_VARIANT)
+    for (u32 x : {v.jw, v.rl, v.rs, v.warps}) h = (h ^ x) * 16777619u;
   return h;
 }
 
+// The bodies that the variants use (range_variants.h): window length and warps per block.
+#define CZ_RANGE_BODIES(X) X(13, 32) X(13, 24) X(12, 32) X(12, 24)
+
 template <int L>
-static cudaError_t launch_t(const RangeArgs& a, int variant, u32 grid, cudaStream_t st) {
-  switch (variant) {
-#define X(id, jw, rl, rs, wp)                                                                               \
-  case id:                                                                                              \
-    k_range<L, jw, rl, rs, wp><<<grid, wp * 32, sizeof(RangeShared<jw, wp>), st>>>(a);            \
-    break;
-    CZ_RANGE_VARIANTS(X)
-#undef X
-    default: return cudaErrorInvalidValue;
+static cudaError_t launch_t(const RangeArgs& a, u32 jw, u32 warps, u32 grid, cudaStream_t st) {
+#define X(j, w)                                                                                    \
+  if (jw == j && warps == w) {                                                                     \
+    k_range<L, j, w><<<grid, w * 32, sizeof(RangeShared<j, w>), st>>>(a);                   \
+    return cudaGetLastError();                                                                     \
   }
-  return cudaGetLastError();
+  CZ_RANGE_BODIES(X)
+#undef X
+  return cudaErrorInvalidValue;
 }
 
-// Variant 0 with fewer than 512 rows to a warp runs with 24 warps per block: such launches spend
-// much of their time opening runs and on the exact path's last seeds, and fewer warps open
-// fewer.  2^28 seeds at 2^40: 115 us with 32 warps, 103 with 24; 2^30: 163 and 152; 2^32: 285
-// and 271; 2^30 at 2^60: 178 and 165.  Long launches need the 32 (2^36: 2.36 and 2.57 ms).
-constexpr int SMALL_VARIANT = 7;
-
-cudaError_t launch_range(const RangeArgs& a, int words, int variant, u32 sm_count, cudaStream_t st) {
-  if (variant == 0 && a.item_limit < 512ull * 32 * sm_count) variant = SMALL_VARIANT;
+cudaError_t launch_range(const RangeArgs& args, int words, int variant, u32 sm_count, cudaStream_t st) {
+  if (variant < 0 || variant >= RANGE_VARIANTS) return cudaErrorInvalidValue;
+  const RangeVariant v = range_pick(variant, args.item_limit, sm_count);
+  RangeArgs a = args;
+  a.rl = v.rl;
+  a.rs = v.rs;
   const u32 grid = (u32)std::max<unsigned long long>(1, std::min<unsigned long long>(sm_count, a.item_limit));
   switch (words) {
-    case 2: return launch_t<2>(a, variant, grid, st);
-    case 3: return launch_t<3>(a, variant, grid, st);
-    case 4: return launch_t<4>(a, variant, grid, st);
+    case 2: return launch_t<2>(a, v.jw, v.warps, grid, st);
+    case 3: return launch_t<3>(a, v.jw, v.warps, grid, st);
+    case 4: return launch_t<4>(a, v.jw, v.warps, grid, st);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -1217,11 +1207,11 @@ cudaError_t launch_range(const RangeArgs& a, int words, int variant, u32 sm_coun
 template <int L>
 static cudaError_t init_t() {
   cudaError_t e = cudaSuccess;
-#define X(id, jw, rl, rs, wp)                                                                                   \
-  if (e == cudaSuccess)                                                                                     \
-    e = cudaFuncSetAttribute(k_range<L, jw, rl, rs, wp>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                             (int)sizeof(RangeShared<jw, wp>));
-  CZ_RANGE_VARIANTS(X)
+#define X(j, w)                                                                                               \
+  if (e == cudaSuccess)                                                                                       \
+    e = cudaFuncSetAttribute(k_range<L, j, w>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
+                             (int)sizeof(RangeShared<j, w>));
+  CZ_RANGE_BODIES(X)
 #undef X
   return e;
 }

@@ -360,11 +360,11 @@ int collatz_server_info(collatz_server *s, collatz_server_info_t *info);
 int collatz_server_stop(collatz_server *s);
 
 /* Kernel choices for the autotuner (no counterpart in the reference).
- *   COLLATZ_MODE_CASES, COLLATZ_MODE_RANGE: variant (block shape, body) of
- *     the cases kernel and of the range kernel for values of three and four
- *     32-bit words;
- *   COLLATZ_MODE_RANGE64: variant of the range kernel for values of two words
- *     (window length, refill thresholds, warps per block);
+ *   COLLATZ_MODE_CASES: variant of the cases kernel;
+ *   COLLATZ_MODE_RANGE, COLLATZ_MODE_RANGE64: variant of the range kernel for
+ *     values of three and four 32-bit words, and of two (window length and
+ *     refill thresholds).  0 to 5 run with 24 warps per block when a launch has
+ *     few rows and with 32 otherwise; 6 and 7 are 0 with 32 and with 24;
  *   COLLATZ_MODE_RANGE64_BITS: the width -- launches whose seeds all have at
  *     most this many bits (0..52; those above 48 count as 48) keep values in
  *     two words, the others in three or four (0: never two).
