@@ -1153,7 +1153,7 @@ cudaError_t cz::range_kernel_launch(collatz_ctx* c, const RangeArgs& a, cudaStre
 static cudaError_t range_enqueue(collatz_ctx* c, const RangeArgs& a, const RangeBufs& b, cudaStream_t s) {
   const size_t rb = sizeof(ReqRec) * std::max(1u, b.n);
   cudaError_t e = cudaMemsetAsync(b.head, 0, sizeof(RangeHead) + rb, s);
-  if (!e && b.stats) e = cudaMemsetAsync(b.stats, 0, 16 * sizeof(unsigned long long), s);
+  if (!e && b.stats) e = cudaMemsetAsync(b.stats, 0, RANGE_STATS * sizeof(unsigned long long), s);
   if (!e) e = range_kernel_launch(c, a, s);
   if (!e) e = launch_range_finish(a, s);
   if (!e) e = cudaMemcpyAsync(b.h_recs, b.recs(), rb, cudaMemcpyDeviceToHost, s);
@@ -1176,7 +1176,7 @@ static int plan_build(collatz_ctx* c, const collatz_range* r, uint32_t n, collat
   CK(c, p->h_recs.ensure(sizeof(ReqRec) * std::max(1u, n)));
   CK(c, p->d_lists.ensure(sizeof(RangeLists)));
   p->stats = range_stats_requested();
-  if (p->stats) CK(c, p->d_stats.ensure(16 * sizeof(unsigned long long)));
+  if (p->stats) CK(c, p->d_stats.ensure(RANGE_STATS * sizeof(unsigned long long)));
   const RangeBufs b{p->d_segs.as<RangeSeg>(), (uint32_t)p->segs.size(), p->items, p->d_range.as<RangeHead>(),
                     p->h_recs.p, n, p->d_lists.as<RangeLists>(),
                     p->stats ? p->d_stats.as<unsigned long long>() : nullptr};
@@ -1231,9 +1231,15 @@ extern "C" int collatz_plan_results(collatz_plan* p, collatz_range_result* out) 
   const ReqRec* h = p->h_recs.as<ReqRec>();
   int status = COLLATZ_OK;
   if (p->stats) {  // diagnostics (COLLATZ_RANGE_STATS=1)
-    unsigned long long st8[16];
-    CK(c, cudaMemcpy(st8, p->d_stats.p, sizeof st8, cudaMemcpyDeviceToHost));
-    fprintf(stderr, "collatz range stats: items=%llu runs=%llu exact_seeds=%llu\n", p->items, st8[0], st8[1]);
+    unsigned long long x[RANGE_STATS];
+    CK(c, cudaMemcpy(x, p->d_stats.p, sizeof x, cudaMemcpyDeviceToHost));
+    fprintf(stderr,
+            "collatz range stats: items=%llu runs=%llu entries=%llu windows=%llu passes=%llu screened=%llu "
+            "screen_windows=%llu exact_seeds=%llu run_pairs=%llu offers=%llu scouts=%llu warp_cycles: windows=%llu "
+            "entries=%llu runs=%llu screen=%llu exact=%llu all=%llu\n",
+            p->items, x[RS_RUNS], x[RS_ENTRIES], x[RS_WINDOWS], x[RS_PASSES], x[RS_SCREENED], x[RS_SCREEN_WINDOWS],
+            x[RS_EXACT], x[RS_RUN_PAIRS], x[RS_OFFERS], x[RS_SCOUTS], x[RS_CYCLES_WINDOWS], x[RS_CYCLES_ENTRIES],
+            x[RS_CYCLES_RUNS], x[RS_CYCLES_SCREEN], x[RS_CYCLES_EXACT], x[RS_CYCLES]);
   }
   for (uint32_t i = 0; i < p->n; i++) {
     rec_to_range_result(h[i], &out[i]);

@@ -132,6 +132,27 @@ struct RangeLists {
   WidenEntry widen[WIDEN_CAP];
 };
 
+// What the diagnostics form of the range kernel counts.
+enum RangeStat : int {
+  RS_RUNS,            // runs of rows opened
+  RS_ENTRIES,         // table entries (or integers) handed to lanes
+  RS_WINDOWS,         // windows of the window loop, by lanes with a seed
+  RS_PASSES,          // groups of four windows of a warp
+  RS_SCREENED,        // seeds that reached a limit and were screened
+  RS_SCREEN_WINDOWS,  // their windows in the screen
+  RS_EXACT,           // seeds on the exact path
+  RS_RUN_PAIRS,       // their run pairs
+  RS_OFFERS,          // offers of a maximum
+  RS_SCOUTS,          // head starts of a request's maxima
+  RS_CYCLES_WINDOWS,  // clock cycles of all warps in the window loop,
+  RS_CYCLES_ENTRIES,  // handing out entries,
+  RS_CYCLES_RUNS,     // opening runs (and waiting for the block at the end),
+  RS_CYCLES_SCREEN,   // in the screen,
+  RS_CYCLES_EXACT,    // on the exact path,
+  RS_CYCLES,          // and in all of these
+  RANGE_STATS
+};
+
 struct RangeArgs {
   const RangeEntry* table;        // survivor table of the 2^k sieve
   uint32_t k;
@@ -143,7 +164,7 @@ struct RangeArgs {
   ReqRec* recs;
   uint32_t iter_cap;              // odd/even run pairs per seed before ERR_ITER_CAP
   uint32_t negative;              // 1: the negative-integer variant (a table built for it)
-  unsigned long long* stats;      // diagnostics: [0] runs of rows, [1] seeds on the exact path; may be null
+  unsigned long long* stats;      // diagnostics counts (RangeStat); null: the kernel without them
   uint32_t seed_bits;             // bit length of the launch's largest seed (0: not known)
   uint32_t rl = 0, rs = 0;        // the variant's thresholds (range_variants.h), set by launch_range
   uint32_t one = 1, mone = ~0u, eight = 8;  // 1, -1 and 8, unknown to the compiler (range.cu: window)

@@ -175,6 +175,7 @@ struct ExactSeed {
              // variant, back at its start; EX_CAP: ST_CAP steps
   u32 st;    // stopping time
   u32 E[4];  // excursion
+  u32 pairs; // run pairs taken
 };
 
 // Runs the seeds n of all lanes together (lanes with have = false idle): odd runs of at most
@@ -183,7 +184,7 @@ struct ExactSeed {
 __device__ __forceinline__ ExactSeed exact_run(u32 n0, u32 n1, u32 n2, bool have, bool neg) {
   ExactSeed R;
   R.how = EX_NONE;
-  R.st = 0;
+  R.st = R.pairs = 0;
   R.E[0] = n0;
   R.E[1] = n1;
   R.E[2] = n2;
@@ -199,6 +200,7 @@ __device__ __forceinline__ ExactSeed exact_run(u32 n0, u32 n1, u32 n2, bool have
 #pragma unroll 1
   while (__any_sync(FULL, alive)) {
     if (alive) {
+      R.pairs++;
       const u32 a = ctz32(v0 | 0x80u);
       odd_run4(v0, v1, v2, v3, a, pow3_le7(a));
       u32 x0, x1, x2, x3;  // the value
@@ -277,10 +279,11 @@ __device__ __forceinline__ void offer(const RangeArgs& A, bool lead, const Range
 // The exact path for the warp's queued seeds e (n limbs 0..2, request), one per
 // lane with have: failures, widening and errors are recorded, and of the seeds of
 // one request that may raise a maximum only the best is offered (larger, or equal
-// with a smaller seed).
-__device__ __forceinline__ void exact_seeds(const RangeArgs& A, uint4 e, bool have) {
+// with a smaller seed).  Adds to the lane's run pairs and to the warp's offers.
+__device__ __forceinline__ void exact_seeds(const RangeArgs& A, uint4 e, bool have, u32& pairs, u32& offers) {
   const u32 lane = lane_id();
   const ExactSeed R = exact_run(e.x, e.y, e.z, have, A.negative != 0);
+  pairs += R.pairs;
   ReqRec* rec = A.recs + e.w;
   bool ps = false, pe = false;
   if (R.how == EX_OK) {
@@ -316,9 +319,11 @@ __device__ __forceinline__ void exact_seeds(const RangeArgs& A, uint4 e, bool ha
 #pragma unroll 1
     for (u32 kind = 0; kind < 2; kind++) {
       const u32 set = kind ? ce : cs;
-      if (set)
+      if (set) {
+        offers++;
         offer(A, lane == (u32)__ffs(set) - 1,
               RangeCand{req, kind, R.st, 0u, {R.E[0], R.E[1], R.E[2], R.E[3]}, {e.x, e.y, e.z, 0u}});
+      }
     }
     pm &= ~__ballot_sync(FULL, in);
   }
@@ -663,9 +668,9 @@ __device__ __forceinline__ uint4 seed_at(uint4 b, u32 g, u32 shift, u32 mul) {
 // output under their requests' keys as they are now.  Windows from the seed's start
 // with four words, the excursion bounded window by window by its own largest D, so that
 // what the window loop's coarser limits stop (a bit of slack and the words' width among
-// them) seldom goes on to the exact path.
+// them) seldom goes on to the exact path.  Adds to the lane's windows.
 template <int L, int JW, class SH>
-__device__ __forceinline__ bool screen(const SH& S, const RangeArgs& A, uint4 e, bool have) {
+__device__ __forceinline__ bool screen(const SH& S, const RangeArgs& A, uint4 e, bool have, u32& windows) {
   const u128 n = ((u128)e.z << 64) | ((u64)e.y << 32) | e.x;
   const ReqRec* r = A.recs + e.w;
   const ull sk = have ? *(volatile const ull*)&r->st_key : 0ull, ek = have ? *(volatile const ull*)&r->e_key : 0ull;
@@ -682,6 +687,7 @@ __device__ __forceinline__ bool screen(const SH& S, const RangeArgs& A, uint4 e,
       exact = true;
       alive = false;
     }
+    windows += alive;
     const u32 t = window<L, JW>(y, P, S, A.mone);
     P &= 0xFFFFu;
     if (t & 0x8000u) alive = false;
@@ -726,8 +732,9 @@ __device__ __forceinline__ ulonglong2 scout(const SH& S, const RangeArgs& A, u32
 
 // The kernel.  It makes no function calls: with one, the compiler takes the warp to be
 // possibly diverged at every vote and spends three instructions on each.  L: words of a value; JW:
-// window length; WARPS per block, one block per SM.
-template <int L, int JW, int WARPS>
+// window length; WARPS per block, one block per SM; STATS: the diagnostics form, which counts into
+// A.stats (RangeStat).
+template <int L, int JW, int WARPS, bool STATS>
 __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__ RangeArgs A) {
   typedef RangeShared<JW, WARPS> Shared;
   Shared& S = *reinterpret_cast<Shared*>(range_smem);
@@ -775,6 +782,15 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
   cp_async_wait_all();
   __syncthreads();
 
+  ull xs[RANGE_STATS] = {}, xt = STATS ? clock64() : 0;  // STATS: counts; the clock at the last look
+  auto clocked = [&](int what) {  // the cycles since then
+    if (STATS) {
+      const ull t = clock64();
+      xs[what] += t - xt;
+      xs[RS_CYCLES] += t - xt;
+      xt = t;
+    }
+  };
   u32 slow = 0, ex = 0;             // seeds queued for the screen and for the exact path
   u32 ring = FULL, next = 0, ents = 0;  // runs begun less one; entries of the current run handed out, of all
   int thr = 0;                      // idle lanes that call for new entries
@@ -831,7 +847,13 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
         const u32 cnt = min(slow, 32u);
         slow -= cnt;
         const uint4 e = lane < cnt ? W.slow[slow + lane] : make_uint4(0u, 0u, 0u, 0u);
-        const bool on = screen<L, JW>(S, A, e, lane < cnt);
+        u32 nw = 0;
+        const bool on = screen<L, JW>(S, A, e, lane < cnt, nw);
+        if (STATS) {
+          xs[RS_SCREENED] += lane < cnt;
+          xs[RS_SCREEN_WINDOWS] += nw;
+          clocked(RS_CYCLES_SCREEN);
+        }
         const u32 b = __ballot_sync(FULL, on);
         if (on) W.exact[ex + __popc(b & ((1u << lane) - 1u))] = e;
         ex += __popc(b);
@@ -840,8 +862,14 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
       if (ex >= 32u || end) {
         const u32 cnt = min(ex, 32u);
         ex -= cnt;
-        exact_seeds(A, lane < cnt ? W.exact[ex + lane] : make_uint4(0u, 0u, 0u, 0u), lane < cnt);
-        if (A.stats && lane == 0) atomicAdd(&A.stats[1], (ull)cnt);
+        u32 np = 0, no = 0;
+        exact_seeds(A, lane < cnt ? W.exact[ex + lane] : make_uint4(0u, 0u, 0u, 0u), lane < cnt, np, no);
+        if (STATS) {
+          xs[RS_EXACT] += lane < cnt;
+          xs[RS_RUN_PAIRS] += np;
+          xs[RS_OFFERS] += lane ? 0 : no;
+          clocked(RS_CYCLES_EXACT);
+        }
       }
 #pragma unroll
       for (int i = 0; i < L; i++) {
@@ -936,10 +964,12 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
           }
           limits(W.lim, W.elim, W.ud, cu.small);
           take_next();
+          if (STATS) xs[RS_ENTRIES]++;
         }
         cnt = __reduce_add_sync(FULL, cnt);
         if (lane == 0) W.acc_seeds += cnt;
         next += min(__popc(idle), ents - next);
+        clocked(RS_CYCLES_ENTRIES);
       } else {
         // ---- the next run ----
         cp_async_wait_all();
@@ -968,6 +998,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
             W.exact[lane] = e;
             ex = __popc(__ballot_sync(FULL, have));
             end = true;
+            clocked(RS_CYCLES_RUNS);
             continue;
           }
           thr = 32;  // no more runs: the lanes finish what they have
@@ -996,6 +1027,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
             const bool kept = nx.kind == 0 || !nx.mod9 || (((A.negative ? KEEP9N : KEEP9) >> (u32)((nx.q_lo + lane) % 9u)) & 1u);
             const ulonglong2 found = scout<L, JW>(S, A, y4, D0, nx.lgn, nx.kind ? 0 : (int)A.k, have && kept);
             ReqRec* r = A.recs + nx.req;
+            if (STATS) xs[RS_SCOUTS] += lane == 0;
             if (lane == 0) {
               atomicMax(&r->st_key, found.x);
               atomicMax(&r->e_key, found.y);
@@ -1024,7 +1056,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
           }
           __syncwarp();
           stage_next(S, W, ring, A, lane, nwarps, first);
+          if (STATS) xs[RS_RUNS] += lane == 0;
         }
+        clocked(RS_CYCLES_RUNS);
       }
       if ((int)__popc(__ballot_sync(FULL, ti >= te)) >= thr) continue;
     }
@@ -1033,10 +1067,15 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
     __syncwarp();
     while (!__any_sync(FULL, (int)P < 0)) {
 #pragma unroll
-      for (int i = 0; i < 4; i++) hot_step<L, JW>(y, yb, p4, g, P, Pn, ud, ti, S, cls, A.one, A.mone, A.eight);
+      for (int i = 0; i < 4; i++) {
+        if (STATS) xs[RS_WINDOWS] += ti < te && (int)P >= 0;
+        hot_step<L, JW>(y, yb, p4, g, P, Pn, ud, ti, S, cls, A.one, A.mone, A.eight);
+      }
+      if (STATS) xs[RS_PASSES] += lane == 0;
       ti = min(ti, te);  // (an idle lane stays within the table's margin)
       if ((int)__popc(__ballot_sync(FULL, ti >= te)) >= thr) break;
     }
+    clocked(RS_CYCLES_WINDOWS);
     // ---- the seeds at a limit go to the exact path (rare) ----
     if (__any_sync(FULL, (int)P < 0)) {
       const bool bad = (int)P < 0 && ti < te;
@@ -1055,7 +1094,11 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
     if (W.acc_seeds) atomicAdd(&A.recs[W.req].seeds, W.acc_seeds);
     atomicAdd(&A.recs[W.req].items_done, W.acc_rows);
   }
-  if (A.stats && lane == 0) atomicAdd(&A.stats[0], (ull)ring);
+  if (STATS) {
+#pragma unroll
+    for (int i = 0; i < RANGE_STATS; i++)
+      if (xs[i] && (i < RS_CYCLES_WINDOWS || lane == 0)) atomicAdd(&A.stats[i], xs[i]);
+  }
 }
 
 // ------------------------------------------------------------------
@@ -1179,9 +1222,13 @@ uint32_t range_variant_rev() {
 
 template <int L>
 static cudaError_t launch_t(const RangeArgs& a, u32 jw, u32 warps, u32 grid, cudaStream_t st) {
+  if (a.stats) {  // diagnostics: the long launches' body
+    k_range<L, 13, 32, true><<<grid, 32 * 32, sizeof(RangeShared<13, 32>), st>>>(a);
+    return cudaGetLastError();
+  }
 #define X(j, w)                                                                                    \
   if (jw == j && warps == w) {                                                                     \
-    k_range<L, j, w><<<grid, w * 32, sizeof(RangeShared<j, w>), st>>>(a);                   \
+    k_range<L, j, w, false><<<grid, w * 32, sizeof(RangeShared<j, w>), st>>>(a);                   \
     return cudaGetLastError();                                                                     \
   }
   CZ_RANGE_BODIES(X)
@@ -1209,10 +1256,13 @@ static cudaError_t init_t() {
   cudaError_t e = cudaSuccess;
 #define X(j, w)                                                                                               \
   if (e == cudaSuccess)                                                                                       \
-    e = cudaFuncSetAttribute(k_range<L, j, w>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
+    e = cudaFuncSetAttribute(k_range<L, j, w, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
                              (int)sizeof(RangeShared<j, w>));
   CZ_RANGE_BODIES(X)
 #undef X
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_range<L, 13, 32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(RangeShared<13, 32>));
   return e;
 }
 
