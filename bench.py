@@ -45,10 +45,11 @@ UNIT = "seeds/s"
 # Algorithmic 32-bit integer operations per surviving seed with values of W words:
 # the step to the lane's next block (W adds), then per window W shifts, W
 # multiply-adds and 7 more (table index, the entry's three fields, the update and the
-# two tests of the coefficient).  Windows per seed: counted by a diagnostics build of
-# the kernel on the workload.
+# two tests of the coefficient).  W is the width that the launch ran with, the windows per
+# seed are counted on a host sample of the workload's seeds.
 OPS_WINDOW = 7
-WORK_MODEL = {"block": {"words": 2, "windows": 1.81}, "frontier": {"words": 3, "windows": 1.77}}
+WINDOW_STEPS = 13
+WINDOW_SAMPLE = 20000
 # Counters of one range-kernel launch taken with ncu, valid only for the
 # sources of the kernel they were captured from: `src` is
 # kernel_source_hash(workload) at capture time (the kernel's own file and the
@@ -82,6 +83,58 @@ def kernel_source_hash(workload: str) -> str:
         with open(os.path.join(ROOT, "collatz_b200", "csrc", name), "rb") as f:
             h.update(f.read())
     return h.hexdigest()[:16]
+
+
+def windows_per_seed(offset: int, size: int, k: int, samples: int = WINDOW_SAMPLE) -> float:
+    """Windows of 13 steps that a surviving seed of [offset, offset + size) takes after its k-step
+    jump, until one in which its coefficient 3^F / 2^i is known to fall below 1 (range.cu: windows);
+    the mean over a fixed pseudo-random sample.  D = 485 F - 306 i is positive exactly while the
+    coefficient is above 1."""
+    import random
+    rng = random.Random(13)
+    mask = (1 << WINDOW_STEPS) - 1
+    entries = {}
+
+    def entry(r):
+        if r not in entries:
+            x, f, d, low = r, 0, 0, 0
+            for _ in range(WINDOW_STEPS):
+                if x & 1:
+                    x, f, d = (3 * x + 1) >> 1, f + 1, d + 179
+                else:
+                    x, d = x >> 1, d - 306
+                low = min(low, d)
+            entries[r] = x, f, 128 * min(-low >> 7, 15)
+        return entries[r]
+
+    windows = taken = 0
+    while taken < samples:
+        y, f, d = rng.getrandbits(k), 0, 0
+        for _ in range(k):
+            if y & 1:
+                y, f, d = (3 * y + 1) >> 1, f + 1, d + 179
+            else:
+                y, d = y >> 1, d - 306
+            if d < 0:
+                break
+        if d < 0:
+            continue  # not kept by the sieve
+        x = ((offset >> k) + rng.randrange(max(1, size >> k))) * 3 ** f + y
+        taken += 1
+        while True:
+            t, g, low = entry(x & mask)
+            windows += 1
+            fell = d < low
+            d += 485 * g - 306 * WINDOW_STEPS
+            if fell or d < 0:
+                break
+            x = (x >> WINDOW_STEPS) * 3 ** g + t
+    return windows / samples
+
+
+def two_word_bits(v) -> int:
+    """The context's width: launches whose seeds have at most this many bits run on two words."""
+    return v.autotune(range_mode=False, cases_mode=False)["range64_bits"]
 
 
 def dist_env():
@@ -507,14 +560,16 @@ def run_served(v, capacity: float, load: float = 0.7, duration: float = 1.0, see
 
 
 def roofline(workload: str, base: int, k: int, survivors: int, mean_ms: float, size: int, sm_count: int,
-             sm_mhz: float, ipk: dict) -> dict:
+             sm_mhz: float, ipk: dict, two_word_bits: int) -> dict:
     """Integer roofline of one k_range launch: algorithmic 32-bit operations
-    (WORK_MODEL) per second of device time, against the measured integer peak at the
+    (OPS_WINDOW) per second of device time, against the measured integer peak at the
     sampled SM clock.  ncu counters are attached only while the kernel sources still
     hash to those they were captured from."""
-    m = WORK_MODEL[workload]
-    ops_per_window = 2 * m["words"] + OPS_WINDOW
-    ops_per_seed = m["words"] + m["windows"] * ops_per_window
+    bits = (base + size - 1).bit_length()
+    words = 2 if bits <= two_word_bits else 3 if bits <= 80 else 4
+    windows = windows_per_seed(base, size, k)
+    ops_per_window = 2 * words + OPS_WINDOW
+    ops_per_seed = words + windows * ops_per_window
     achieved = survivors * ops_per_seed / (mean_ms / 1e3) / 1e12
     peak = ipk[1]["ops_per_clk_sm"] * sm_count * sm_mhz * 1e6 / 1e12
     issue_peak = sm_count * 128 * sm_mhz * 1e6 / 1e12
@@ -530,8 +585,8 @@ def roofline(workload: str, base: int, k: int, survivors: int, mean_ms: float, s
                            f"kernel sources {cap['src']}" + (f" x {max(1, size >> k)} blocks" if cap["per"] != "launch"
                                                              else "")) if valid else
          f"null: the kernel sources ({src}) changed since the last ncu capture ({cap['src']})",
-         "model": f"{ops_per_seed:.1f} algorithmic 32-bit ops per surviving seed ({m['words']} + {ops_per_window} x "
-                  f"{m['windows']} windows of 13 steps) x {survivors} seeds per launch",
+         "model": f"{ops_per_seed:.1f} algorithmic 32-bit ops per surviving seed ({words} + {ops_per_window} x "
+                  f"{windows:.2f} windows of {WINDOW_STEPS} steps, counted on a host sample of {WINDOW_SAMPLE} seeds) x {survivors} seeds per launch",
          "peak_basis": f"measured integer peak (collatz_int_peak mix 1: funnel shift, 3-input add, multiply-add "
                        f"chains on every SM): {ipk[1]['ops_per_clk_sm']:.1f} ops per SM clock x {sm_count} SMs x "
                        f"{sm_mhz:.0f} MHz (sampled median SM clock); MEASURED_PEAKS.json has no integer peak",
@@ -591,7 +646,7 @@ def run_frontier(local: int, stream, flush, sm_count: int, ipk: dict, steps: int
         plan.close()
         mean_ms = sum(ms) / len(ms)
         roof = roofline("frontier", wl["offset"], wl["k"], res.seeds_checked, mean_ms, size, sm_count,
-                        clocks.get("sm_mhz") or 1965.0, ipk)
+                        clocks.get("sm_mhz") or 1965.0, ipk, two_word_bits(fv))
         return {"workload": f"range [2^60, 2^60 + 2^40), k={wl['k']} sieve (2^34-bit bit array + class-major "
                             "survivor table resident in HBM) + mod-9, 128-bit limbs widening to 192/256, plain kernel",
                 "steps": steps, "warmup": warmup, "ms_per_step": mean_ms, "seeds_per_s": size / (mean_ms / 1e3),
@@ -795,7 +850,7 @@ def main():
         # kernel mix's operations per SM clock, scaled to the clock sampled under load
         ipk = {m: v.int_peak(m) for m in (1, 0)}
         roof = roofline(args.workload, base, ksv, res.seeds_checked, sum(ms) / len(ms), size, sm_count, sm_mhz,
-                        ipk)
+                        ipk, two_word_bits(v))
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": 1e3 * dev_s / args.steps, "higher_is_better": True,
