@@ -25,9 +25,9 @@ struct CasesArgs {
   unsigned long long* overflow_count;
   uint32_t iter_cap;       // checkpoints per seed before ERR_ITER_CAP
   uint32_t multi;          // line batch: base limb 3 = bigindex | line << 8, rec[line] per line
-  uint32_t unit = 0;       // of the table-driven kernel's limits (case_limits.h), set by its launcher
   uint32_t four = 4, p5 = 1u << 5, p29 = 1u << 29;  // unknown to the compiler (cases_win.cu: additions and
                                                     // shifts on the multiply-add pipe)
+  uint32_t unit = 0;       // of the table-driven kernel's limits (case_limits.h), set by its launcher
 };
 int cases_variants();
 cudaError_t launch_cases(const CasesArgs& a, int variant, uint32_t grid, cudaStream_t st);
@@ -166,8 +166,8 @@ struct RangeArgs {
   uint32_t negative;              // 1: the negative-integer variant (a table built for it)
   unsigned long long* stats;      // diagnostics counts (RangeStat); null: the kernel without them
   uint32_t seed_bits;             // bit length of the launch's largest seed (0: not known)
-  uint32_t rl = 0, rs = 0;        // the variant's thresholds (range_variants.h), set by launch_range
   uint32_t one = 1, mone = ~0u, eight = 8;  // 1, -1 and 8, unknown to the compiler (range.cu: window)
+  uint32_t rl = 0, rs = 0;        // the variant's thresholds (range_variants.h), set by launch_range
 };
 // Largest N that runs the kernel with run pairs from a table (cases_win.cu), whose values go to the
 // exact path from 2^71 on: at N = 48 a line of 304 724 seeds took 0.156 ms with it and 0.392

@@ -175,16 +175,18 @@ struct ExactSeed {
              // variant, back at its start; EX_CAP: ST_CAP steps
   u32 st;    // stopping time
   u32 E[4];  // excursion
-  u32 pairs; // run pairs taken
+  u32 pairs; // STATS: run pairs taken
 };
 
 // Runs the seeds n of all lanes together (lanes with have = false idle): odd runs of at most
 // 7 steps and even runs of at most 31 on four limbs.  Written for size: the code is
 // fetched anew by every launch, and few seeds come here.
+template <bool STATS>
 __device__ __forceinline__ ExactSeed exact_run(u32 n0, u32 n1, u32 n2, bool have, bool neg) {
   ExactSeed R;
   R.how = EX_NONE;
-  R.st = R.pairs = 0;
+  R.st = 0;
+  if constexpr (STATS) R.pairs = 0;
   R.E[0] = n0;
   R.E[1] = n1;
   R.E[2] = n2;
@@ -200,7 +202,7 @@ __device__ __forceinline__ ExactSeed exact_run(u32 n0, u32 n1, u32 n2, bool have
 #pragma unroll 1
   while (__any_sync(FULL, alive)) {
     if (alive) {
-      R.pairs++;
+      if constexpr (STATS) R.pairs++;
       const u32 a = ctz32(v0 | 0x80u);
       odd_run4(v0, v1, v2, v3, a, pow3_le7(a));
       u32 x0, x1, x2, x3;  // the value
@@ -279,11 +281,12 @@ __device__ __forceinline__ void offer(const RangeArgs& A, bool lead, const Range
 // The exact path for the warp's queued seeds e (n limbs 0..2, request), one per
 // lane with have: failures, widening and errors are recorded, and of the seeds of
 // one request that may raise a maximum only the best is offered (larger, or equal
-// with a smaller seed).  Adds to the lane's run pairs and to the warp's offers.
-__device__ __forceinline__ void exact_seeds(const RangeArgs& A, uint4 e, bool have, u32& pairs, u32& offers) {
+// with a smaller seed).  STATS: counts the lane's run pairs and the warp's offers.
+template <bool STATS>
+__device__ __forceinline__ void exact_seeds(const RangeArgs& A, uint4 e, bool have, ull* xs) {
   const u32 lane = lane_id();
-  const ExactSeed R = exact_run(e.x, e.y, e.z, have, A.negative != 0);
-  pairs += R.pairs;
+  const ExactSeed R = exact_run<STATS>(e.x, e.y, e.z, have, A.negative != 0);
+  if constexpr (STATS) xs[RS_RUN_PAIRS] += R.pairs;
   ReqRec* rec = A.recs + e.w;
   bool ps = false, pe = false;
   if (R.how == EX_OK) {
@@ -319,11 +322,10 @@ __device__ __forceinline__ void exact_seeds(const RangeArgs& A, uint4 e, bool ha
 #pragma unroll 1
     for (u32 kind = 0; kind < 2; kind++) {
       const u32 set = kind ? ce : cs;
-      if (set) {
-        offers++;
+      if (STATS && set && lane == 0) xs[RS_OFFERS]++;
+      if (set)
         offer(A, lane == (u32)__ffs(set) - 1,
               RangeCand{req, kind, R.st, 0u, {R.E[0], R.E[1], R.E[2], R.E[3]}, {e.x, e.y, e.z, 0u}});
-      }
     }
     pm &= ~__ballot_sync(FULL, in);
   }
@@ -668,9 +670,9 @@ __device__ __forceinline__ uint4 seed_at(uint4 b, u32 g, u32 shift, u32 mul) {
 // output under their requests' keys as they are now.  Windows from the seed's start
 // with four words, the excursion bounded window by window by its own largest D, so that
 // what the window loop's coarser limits stop (a bit of slack and the words' width among
-// them) seldom goes on to the exact path.  Adds to the lane's windows.
-template <int L, int JW, class SH>
-__device__ __forceinline__ bool screen(const SH& S, const RangeArgs& A, uint4 e, bool have, u32& windows) {
+// them) seldom goes on to the exact path.  STATS: counts the lane's windows.
+template <int L, int JW, bool STATS, class SH>
+__device__ __forceinline__ bool screen(const SH& S, const RangeArgs& A, uint4 e, bool have, ull* xs) {
   const u128 n = ((u128)e.z << 64) | ((u64)e.y << 32) | e.x;
   const ReqRec* r = A.recs + e.w;
   const ull sk = have ? *(volatile const ull*)&r->st_key : 0ull, ek = have ? *(volatile const ull*)&r->e_key : 0ull;
@@ -687,7 +689,7 @@ __device__ __forceinline__ bool screen(const SH& S, const RangeArgs& A, uint4 e,
       exact = true;
       alive = false;
     }
-    windows += alive;
+    if constexpr (STATS) xs[RS_SCREEN_WINDOWS] += alive;
     const u32 t = window<L, JW>(y, P, S, A.mone);
     P &= 0xFFFFu;
     if (t & 0x8000u) alive = false;
@@ -782,9 +784,13 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
   cp_async_wait_all();
   __syncthreads();
 
-  ull xs[RANGE_STATS] = {}, xt = STATS ? clock64() : 0;  // STATS: counts; the clock at the last look
+  ull xs[STATS ? RANGE_STATS : 1], xt;  // STATS: counts; the clock at the last look
+  if constexpr (STATS) {
+    for (ull& x : xs) x = 0;
+    xt = clock64();
+  }
   auto clocked = [&](int what) {  // the cycles since then
-    if (STATS) {
+    if constexpr (STATS) {
       const ull t = clock64();
       xs[what] += t - xt;
       xs[RS_CYCLES] += t - xt;
@@ -847,11 +853,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
         const u32 cnt = min(slow, 32u);
         slow -= cnt;
         const uint4 e = lane < cnt ? W.slow[slow + lane] : make_uint4(0u, 0u, 0u, 0u);
-        u32 nw = 0;
-        const bool on = screen<L, JW>(S, A, e, lane < cnt, nw);
-        if (STATS) {
+        const bool on = screen<L, JW, STATS>(S, A, e, lane < cnt, xs);
+        if constexpr (STATS) {
           xs[RS_SCREENED] += lane < cnt;
-          xs[RS_SCREEN_WINDOWS] += nw;
           clocked(RS_CYCLES_SCREEN);
         }
         const u32 b = __ballot_sync(FULL, on);
@@ -862,14 +866,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
       if (ex >= 32u || end) {
         const u32 cnt = min(ex, 32u);
         ex -= cnt;
-        u32 np = 0, no = 0;
-        exact_seeds(A, lane < cnt ? W.exact[ex + lane] : make_uint4(0u, 0u, 0u, 0u), lane < cnt, np, no);
-        if (STATS) {
-          xs[RS_EXACT] += lane < cnt;
-          xs[RS_RUN_PAIRS] += np;
-          xs[RS_OFFERS] += lane ? 0 : no;
-          clocked(RS_CYCLES_EXACT);
-        }
+        exact_seeds<STATS>(A, lane < cnt ? W.exact[ex + lane] : make_uint4(0u, 0u, 0u, 0u), lane < cnt, xs);
+        // (in every form: without this branch 2^32 seeds with k 16 took 406 us and not 397)
+        if (A.stats && lane == 0) atomicAdd(&A.stats[RS_EXACT], (ull)cnt);
+        clocked(RS_CYCLES_EXACT);
       }
 #pragma unroll
       for (int i = 0; i < L; i++) {
@@ -964,7 +964,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
           }
           limits(W.lim, W.elim, W.ud, cu.small);
           take_next();
-          if (STATS) xs[RS_ENTRIES]++;
+          if constexpr (STATS) xs[RS_ENTRIES]++;
         }
         cnt = __reduce_add_sync(FULL, cnt);
         if (lane == 0) W.acc_seeds += cnt;
@@ -1027,7 +1027,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
             const bool kept = nx.kind == 0 || !nx.mod9 || (((A.negative ? KEEP9N : KEEP9) >> (u32)((nx.q_lo + lane) % 9u)) & 1u);
             const ulonglong2 found = scout<L, JW>(S, A, y4, D0, nx.lgn, nx.kind ? 0 : (int)A.k, have && kept);
             ReqRec* r = A.recs + nx.req;
-            if (STATS) xs[RS_SCOUTS] += lane == 0;
+            if constexpr (STATS) xs[RS_SCOUTS] += lane == 0;
             if (lane == 0) {
               atomicMax(&r->st_key, found.x);
               atomicMax(&r->e_key, found.y);
@@ -1056,7 +1056,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
           }
           __syncwarp();
           stage_next(S, W, ring, A, lane, nwarps, first);
-          if (STATS) xs[RS_RUNS] += lane == 0;
         }
         clocked(RS_CYCLES_RUNS);
       }
@@ -1068,10 +1067,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
     while (!__any_sync(FULL, (int)P < 0)) {
 #pragma unroll
       for (int i = 0; i < 4; i++) {
-        if (STATS) xs[RS_WINDOWS] += ti < te && (int)P >= 0;
+        if constexpr (STATS) xs[RS_WINDOWS] += ti < te && (int)P >= 0;
         hot_step<L, JW>(y, yb, p4, g, P, Pn, ud, ti, S, cls, A.one, A.mone, A.eight);
       }
-      if (STATS) xs[RS_PASSES] += lane == 0;
+      if constexpr (STATS) xs[RS_PASSES] += lane == 0;
       ti = min(ti, te);  // (an idle lane stays within the table's margin)
       if ((int)__popc(__ballot_sync(FULL, ti >= te)) >= thr) break;
     }
@@ -1094,7 +1093,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_range(const __grid_constant__
     if (W.acc_seeds) atomicAdd(&A.recs[W.req].seeds, W.acc_seeds);
     atomicAdd(&A.recs[W.req].items_done, W.acc_rows);
   }
-  if (STATS) {
+  if (A.stats && lane == 0) atomicAdd(&A.stats[RS_RUNS], (ull)(ring + 1u));
+  if constexpr (STATS) {
 #pragma unroll
     for (int i = 0; i < RANGE_STATS; i++)
       if (xs[i] && (i < RS_CYCLES_WINDOWS || lane == 0)) atomicAdd(&A.stats[i], xs[i]);
