@@ -36,13 +36,6 @@ static void limbs4(u128 x, uint32_t* w) {
   for (int i = 0; i < 4; i++) w[i] = (uint32_t)(x >> (32 * i));
 }
 
-static int cases_grid(collatz_ctx* c, int variant) {
-  int bps = 0;
-  cudaError_t e = cases_occupancy(variant, &bps);
-  if (e != cudaSuccess || bps <= 0) bps = 1;
-  return bps * c->sm_count;
-}
-
 void rec_to_range_result(const ReqRec& r, collatz_range_result* out) {
   std::memset(out, 0, sizeof *out);
   out->seeds_checked = r.seeds;
@@ -170,7 +163,6 @@ int lower_range(collatz_ctx* c, const collatz_range& r, uint32_t req, const Rang
       g.nq = take;
       g.s_lo = s_lo;
       g.s_hi = s_hi;
-      g.ipq = ipq;
       g.req = req;
       g.kind = 0;
       g.qstride = (uint16_t)stride;
@@ -463,7 +455,7 @@ extern "C" int collatz_verify_pairs(collatz_ctx* c, uint32_t bigindex, const uin
     CK(c, cudaMemsetAsync(c->d_counter.p, 0, sizeof(uint32_t), c->stream));
     CasesArgs a = case_args(c, c->d_pairs[0].as<uint32_t>(), npairs, (int)bigindex);
     CK(c, cudaEventRecord(c->ev[0], c->stream));
-    CK(c, launch_cases(a, c->cases_variant, cases_grid(c, c->cases_variant), c->stream));
+    CK(c, launch_cases(a, c->cases_variant, (uint32_t)c->sm_count, c->stream));
     CK(c, cudaEventRecord(c->ev[1], c->stream));
   }
   CK(c, cudaStreamSynchronize(c->stream));
@@ -663,7 +655,7 @@ static int run_case_host(collatz_ctx* c, const collatz_case* cs, collatz_case_re
       if (!err) err = cudaEventRecord(e0, c->stream);
       if (!err) {
         CasesArgs a = case_args(c, c->d_pairs[slot].as<uint32_t>(), job.second, -1);
-        err = launch_cases(a, c->cases_variant, cases_grid(c, c->cases_variant), c->stream);
+        err = launch_cases(a, c->cases_variant, (uint32_t)c->sm_count, c->stream);
       }
       if (!err) err = cudaEventRecord(e1, c->stream);
       if (!err) err = cudaEventRecord(kdone[slot], c->stream);
@@ -851,7 +843,7 @@ static int run_case_device(collatz_ctx* c, const collatz_case* cs, collatz_case_
       CK(c, s1_emit(c, R, lo, hi, dp));
       CK(c, cudaMemsetAsync(c->d_counter.p, 0, sizeof(uint32_t), c->stream));
       CasesArgs a = case_args(c, dp, (uint32_t)(hi - lo), -1);
-      CK(c, launch_cases(a, c->cases_variant, cases_grid(c, c->cases_variant), c->stream));
+      CK(c, launch_cases(a, c->cases_variant, (uint32_t)c->sm_count, c->stream));
     }
     CK(c, cudaEventRecord(c->ev[1], c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
@@ -931,9 +923,7 @@ static int batch_pass(collatz_ctx* c, const collatz_case* cases, const std::vect
       CasesArgs a = case_args(c, dp, (uint32_t)(hi - lo), -1);
       a.rec = c->d_recs.as<ReqRec>();
       a.multi = 1;
-      int bps = 0;
-      if (cases_occupancy(c->cases_variant, &bps, true) != cudaSuccess || bps <= 0) bps = 1;
-      CK(c, launch_cases(a, c->cases_variant, (uint32_t)(bps * c->sm_count), c->stream));
+      CK(c, launch_cases(a, c->cases_variant, (uint32_t)c->sm_count, c->stream));
     }
     CK(c, cudaEventRecord(c->ev[1], c->stream));
     CK(c, cudaStreamSynchronize(c->stream));

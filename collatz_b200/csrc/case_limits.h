@@ -16,9 +16,9 @@ constexpr int CP_STEPS = 12;  // most steps of a look-up
 // The limits on values are kept in units of 2^(32 + this), below 2^23 units.  A line whose maximum is
 // below 256 units runs every seed exactly, and so does a seed that reaches 2^23 units: the unit
 // grows with N, so that the largest start of a checkpoint loop, n 1.5^(N - 10) < 2^(1.585 N - 5.8), lies
-// a factor of 2^5 below that.  With 2^48 for every N, 2000 lines of N = 36 took
-// 3.28 ms on the device and 1370 larger ones 7.1, so 1.06 and 2.74.  With units of 2^41 at N = 45, the
-// lines of the largest starts took 0.41 ms and not 0.24.
+// a factor of 2^5 below that, up to N = 45, from where on it is 2^48.  With 2^48 for every N, 2000
+// lines of N = 36 took 3.28 ms on the device and 1370 larger ones 7.1, so 1.06 and 2.74.  With units of
+// 2^41 at N = 45, the lines of the largest starts took 0.41 ms and not 0.24.
 CZ_HD uint32_t line_unit(uint32_t maxbits) {
   const uint32_t top = (maxbits * 317u + 199u) / 200u;  // 1.585 N, rounded up
   return top < 55u ? 0u : top < 71u ? top - 55u : 16u;

@@ -424,41 +424,33 @@ __global__ void __launch_bounds__(CWARPS * 32) k_cases(const CasesArgs A) {
 // Host launcher.
 // ------------------------------------------------------------------
 
-template <int I, int R>
-static cudaError_t launch_cases_t(const CasesArgs& a, u32 grid, cudaStream_t st) {
-  if (a.multi) k_cases<I, R, true><<<grid, CWARPS * 32, 0, st>>>(a);
-  else k_cases<I, R, false><<<grid, CWARPS * 32, 0, st>>>(a);
+// As many blocks as the device holds.
+template <int I, int R, bool M>
+static cudaError_t launch_cases_t(const CasesArgs& a, u32 sm_count, cudaStream_t st) {
+  int bps = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_cases<I, R, M>, CWARPS * 32, 0) != cudaSuccess || bps <= 0) bps = 1;
+  k_cases<I, R, M><<<(u32)bps * sm_count, CWARPS * 32, 0, st>>>(a);
   return cudaGetLastError();
+}
+template <int I, int R>
+static cudaError_t launch_cases_t(const CasesArgs& a, u32 sm_count, cudaStream_t st) {
+  return a.multi ? launch_cases_t<I, R, true>(a, sm_count, st) : launch_cases_t<I, R, false>(a, sm_count, st);
 }
 
 // Variants: checkpoints per pass and refill threshold; variant 4 is the kernel with run
-// pairs from a table (cases_win.cu) for N <= 52, where values up to 2^56 leave few seeds to
-// its exact path, and variant 3 above.
+// pairs from a table (cases_win.cu) for N <= 52, where few seeds start at or rise to the 2^71 from
+// which they take its exact path, and variant 3 above.
 int cases_variants() { return 5; }
 
-cudaError_t launch_cases(const CasesArgs& a, int variant, u32 grid, cudaStream_t st) {
+cudaError_t launch_cases(const CasesArgs& a, int variant, u32 sm_count, cudaStream_t st) {
   // seeds n = base | a << (N - A) lie below 2^N (A = 10)
-  if (variant == 4 && a.mbi + 10u <= CASES_WIN_MAX_BITS) return launch_cases_win(a, st);
+  if (variant == 4 && a.mbi + 10u <= CASES_WIN_MAX_BITS) return launch_cases_win(a, sm_count, st);
   switch (variant) {
-    case 0: return launch_cases_t<1, 1>(a, grid, st);
-    case 1: return launch_cases_t<2, 4>(a, grid, st);
-    case 2: return launch_cases_t<2, 8>(a, grid, st);
-    default: return launch_cases_t<4, 8>(a, grid, st);
+    case 0: return launch_cases_t<1, 1>(a, sm_count, st);
+    case 1: return launch_cases_t<2, 4>(a, sm_count, st);
+    case 2: return launch_cases_t<2, 8>(a, sm_count, st);
+    default: return launch_cases_t<4, 8>(a, sm_count, st);
   }
-}
-
-template <bool M>
-static cudaError_t occupancy_t(int variant, int* bps) {
-  switch (variant) {
-    case 0: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_cases<1, 1, M>, CWARPS * 32, 0);
-    case 1: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_cases<2, 4, M>, CWARPS * 32, 0);
-    case 2: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_cases<2, 8, M>, CWARPS * 32, 0);
-    default: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k_cases<4, 8, M>, CWARPS * 32, 0);
-  }
-}
-
-cudaError_t cases_occupancy(int variant, int* blocks_per_sm, bool multi) {
-  return multi ? occupancy_t<true>(variant, blocks_per_sm) : occupancy_t<false>(variant, blocks_per_sm);
 }
 
 }  // namespace cz

@@ -93,6 +93,8 @@ struct CwShared {
   CwWarp w[WWARPS];
 };
 
+static_assert(sizeof(CwShared) <= MAX_BLOCK_SMEM, "shared memory of a block");
+
 extern __shared__ __align__(16) unsigned char cw_smem[];
 
 __device__ __forceinline__ u32 lds32(u32 at) {
@@ -558,12 +560,8 @@ cudaError_t cases_win_init(cudaStream_t st) {
                    [&] { return mark_table(g_cp_ready, st); });
 }
 
-cudaError_t launch_cases_win(const CasesArgs& a, cudaStream_t st) {
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (!e) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e) return e;
-  const u32 grid = std::min((u32)sms, std::max(1u, a.npairs));
+cudaError_t launch_cases_win(const CasesArgs& a, u32 sm_count, cudaStream_t st) {
+  const u32 grid = std::min(sm_count, std::max(1u, a.npairs));
   CasesArgs b = a;
   b.unit = line_unit(a.mbi + 10u);
   const auto k = b.unit == MAX_UNIT ? (b.multi ? k_cases_win<true, MAX_UNIT> : k_cases_win<false, MAX_UNIT>)

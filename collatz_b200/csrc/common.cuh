@@ -251,6 +251,8 @@ __device__ __forceinline__ void key_decode(ull key, u32* w) {
   }
 }
 
+constexpr size_t MAX_BLOCK_SMEM = 227 * 1024;  // of a block, opted in
+
 // ---------------------------------------------------------------------
 // Record locks with a bounded spin: after LOCK_SPIN_LIMIT attempts the
 // caller gives up and sets ERR_LOCK, so no kernel can wait forever.

@@ -30,11 +30,10 @@ struct CasesArgs {
   uint32_t unit = 0;       // of the table-driven kernel's limits (case_limits.h), set by its launcher
 };
 int cases_variants();
-cudaError_t launch_cases(const CasesArgs& a, int variant, uint32_t grid, cudaStream_t st);
+cudaError_t launch_cases(const CasesArgs& a, int variant, uint32_t sm_count, cudaStream_t st);
 // For every context, before its first launch; the tables are filled by a device's first.  Ends with st idle.
 cudaError_t cases_win_init(cudaStream_t st);
-cudaError_t launch_cases_win(const CasesArgs& a, cudaStream_t st);  // N <= 52
-cudaError_t cases_occupancy(int variant, int* blocks_per_sm, bool multi = false);
+cudaError_t launch_cases_win(const CasesArgs& a, uint32_t sm_count, cudaStream_t st);  // N <= 52
 
 // ---------------- device Step 1 (step1_dev.cu) ----------------
 // A node of search1's tree (cu:497-505): base and number as little-endian
@@ -93,8 +92,7 @@ struct RangeSeg {
   uint32_t q_hi;                  // kind 0: first block, bits 64..95
   uint32_t nq;                    // kind 0: number of blocks
   uint32_t s_lo, s_hi;            // kind 0: survivor index range
-  uint32_t ipq;                   // kind 0: items per block
-  uint32_t req;                   // request index (ReqRec)
+  uint32_t req, pad;              // request index (ReqRec)
   uint16_t kind;
   uint16_t qstride;               // kind 0: 0 or 1: consecutive blocks; 9: the blocks that keep the class
   uint32_t mod9;                  // kind 0: the class (r mod 9); kind 1: 1 to apply the mod-9 sieve
@@ -171,7 +169,8 @@ struct RangeArgs {
 };
 // Largest N that runs the kernel with run pairs from a table (cases_win.cu), whose values go to the
 // exact path from 2^71 on: at N = 48 a line of 304 724 seeds took 0.156 ms with it and 0.392
-// with four limbs, at N = 52 one of 3.75 M seeds 0.274 and 0.578.
+// with four limbs, at N = 52 one of 3.75 M seeds 0.274 and 0.578.  There is no smallest N: the
+// whole tree took 0.17 and 0.22 ms at N = 20, 0.16 and 0.36 at 26, 2.2 and 5.1 at 36, 21 and 59 at 40.
 constexpr uint32_t CASES_WIN_MAX_BITS = 52;
 int range_variants();
 int range64_variants();

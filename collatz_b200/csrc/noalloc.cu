@@ -121,10 +121,8 @@ extern "C" int collatz_verify_pairs_noalloc(collatz_ctx* c, uint32_t bigindex, c
     a.overflow_count = d_ovcount;
     a.iter_cap = c->iter_cap;
     a.multi = 0;
-    int bps = 0;
-    if (cases_occupancy(c->cases_variant, &bps) != cudaSuccess || bps <= 0) bps = 1;
     NA_CK(c, cudaEventRecord(c->ev[0], c->stream));
-    NA_CK(c, launch_cases(a, c->cases_variant, (uint32_t)(bps * c->sm_count), c->stream));
+    NA_CK(c, launch_cases(a, c->cases_variant, (uint32_t)c->sm_count, c->stream));
     NA_CK(c, cudaEventRecord(c->ev[1], c->stream));
   }
   ReqRec r;

@@ -23,12 +23,12 @@
 //     remainder: 0 <= rho_i <= C_i F_i / 3.
 //   * So C_i > 1 keeps T^i(n) above n, and at the first i with C_i < 1, T^i(n) <
 //     n as soon as n > F_i / (3 (1/C_i - 1)); for i < 485 that bound is below
-//     32 900 (the nearest 2^i / 3^F above 1 is 2^401 / 3^253 = 1.0031).  For the
+//     27 100 (the nearest 2^i / 3^F above 1 is 2^401 / 3^253 = 1.0031).  For the
 //     negative variant rho_i is subtracted: C_i < 1 gives T'^i(m) < m at once, and
-//     C_i > 1 keeps T'^i(m) above m when m > F_i / (3 (1 - 1/C_i)), below 48 900
-//     (3^53 / 2^84 = 1.0021).  Seeds of at least 2^16 satisfy both.
+//     C_i > 1 keeps T'^i(m) above m when m > F_i / (3 (1 - 1/C_i)), below 8 600
+//     (3^265 / 2^420 = 1.0105).  Seeds of at least 2^16 satisfy both.
 //   * T^i(n) <= C_i (n + F_i / 3), so D_i / 306 + log2(n) bounds log2 T^i(n) from
-//     above to within 0.0023.
+//     above to within 0.0024.
 // A seed whose D is negative after a window has therefore fallen below its
 // start within it.  Its stopping time is at most the steps taken and its
 // excursion at most what D allowed; both are below the request's running maxima
@@ -43,7 +43,7 @@
 // seed to the widen list, re-run with 6 and then 8 limbs.  A request whose maxima are still zero
 // gets a head start from a run's first seeds (scout).
 //
-// 2^38 seeds at 2^40, k 24: 5.9 ms, against 39 ms with run pairs in each lane.
+// 2^38 seeds at 2^40, k 24: 5.9 ms, against 43 ms with run pairs in each lane.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -97,7 +97,7 @@ constexpr int window_slack(int jw) {
 // (layout 1) f << 3, with f the odd steps and m = floor(-min D_i / 128) of the window's D_i (at
 // most 15; 0 when none is negative): a seed with D < 128 m at the window's start falls
 // below its start inside it.
-constexpr u32 MIN_JW = 11, MAX_JW = 13;  // T^13(r) < 3^13 < 2^21
+constexpr u32 MIN_JW = 12, MAX_JW = 13;  // T^13(r) < 3^13 < 2^21
 constexpr u32 WIN_M = 0x780u;
 __device__ u32 g_win[2][2][MAX_JW - MIN_JW + 1][1u << MAX_JW];
 // The largest D_i of the window, in units of 16, rounded up (for the screen).
@@ -501,7 +501,7 @@ template <int L, int JW>
 __device__ __forceinline__ RunLimits run_limits(ulonglong2 keys, float lgn, int s0) {
   const ull sk = keys.x;
   RunLimits R;
-  // the margins cover the float arithmetic and the 0.0023 of the bound on T^i(n)
+  // the margins cover the float arithmetic and the 0.0024 of the bound on T^i(n)
   R.elim = (int)floorf((float)DB * (key_log2(keys.y) - lgn)) - 2;
   const int lo = (int)floorf((float)DB * ((float)(32 * L - 2) - lgn)) - 2;  // values stay in L words
   R.lim = min(min(R.elim, lo), LIM_MAX) - window_slack(JW) - 1;
@@ -1219,6 +1219,9 @@ uint32_t range_variant_rev() {
 
 // The bodies that the variants use (range_variants.h): window length and warps per block.
 #define CZ_RANGE_BODIES(X) X(13, 32) X(13, 24) X(12, 32) X(12, 24)
+#define X(j, w) static_assert(sizeof(RangeShared<j, w>) <= MAX_BLOCK_SMEM, "shared memory of a block");
+CZ_RANGE_BODIES(X)
+#undef X
 
 template <int L>
 static cudaError_t launch_t(const RangeArgs& a, u32 jw, u32 warps, u32 grid, cudaStream_t st) {
