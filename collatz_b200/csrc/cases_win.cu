@@ -84,7 +84,8 @@ struct CwWarp {
   uint2 slow[64];             // seeds for the exact path: pair, a
   unsigned short q[WQ];       // (slot << 10) | a
   uint4 ring[WR][3];          // base0..1, number0..2, 3^f limbs 0..2, limits, pair, line, limbs above those
-                              // kept (not 0: the pair's seeds all go to the exact path)
+                              // kept (2: of the base, 1: of the values only; the pair's seeds then all go to the
+                              // exact path)
 };
 
 struct CwShared {
@@ -385,7 +386,7 @@ __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_const
           if (lane == 8) R[8] = lim;
           if (lane == 9) R[9] = p;
           if (lane == 10) R[10] = pline;
-          if (lane == 11) R[11] = b2 | n3 | A.pow3[4u * f + 3];
+          if (lane == 11) R[11] = b2 ? 2u : (n3 | A.pow3[4u * f + 3]) != 0;
           if (MULTI && __any_sync(FULL, pline != wline)) {  // seeds are counted per warp until the line changes
             if (lane == 0 && warp_seeds) atomicAdd(&A.rec[wline].seeds, (ull)warp_seeds);
             warp_seeds = 0;
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_const
         npair = r2.y;
         na10 = a;
         nline = r2.z;
-        if (n < 3 && r2.w == 0) {  // v < n can never hold: the reference would loop forever
+        if (n < 3 && r2.w != 2u) {  // v < n can never hold: the reference would loop forever
           atomicOr(&A.rec[nline].errors, ERR_SEED_SMALL);
           w0 = w1 = w2 = 0;
         }
