@@ -124,7 +124,7 @@ static_assert(sizeof(RangeHead) == 64, "RangeHead");
 
 // Lists of a launch; their lengths are in the head.
 constexpr uint32_t WIDEN_CAP = 1u << 16;
-constexpr uint32_t CAND_CAP = 1u << 15;  // candidates beyond it take the record's lock in the kernel
+constexpr uint32_t CAND_CAP = 1u << 16;  // candidates beyond it take the record's lock in the kernel
 struct RangeLists {
   RangeCand cand[CAND_CAP];
   WidenEntry widen[WIDEN_CAP];

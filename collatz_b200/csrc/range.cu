@@ -1155,7 +1155,10 @@ __device__ __noinline__ u32 wide_seed(const WidenEntry& e, bool neg, u32 iter_ca
 __global__ void __launch_bounds__(128) k_range_finish(const __grid_constant__ RangeArgs A) {
   const u32 t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x, lane = lane_id();
   const u32 nc = min(A.head->cands, CAND_CAP), nw = min(A.head->widened, WIDEN_CAP);
-  // candidates still at their record's keys, one lane at a time (record locks)
+  // candidates still at their record's keys: one lane at a time for a request (record locks), the
+  // requests of a warp's lanes side by side.  A batch of small requests has two candidates for each:
+  // 1000 requests of 64 to 256 seeds take 75 us, and took 129 with one lane at a time for all; 20 000 take
+  // 0.22 ms and took 0.52 (with half the list's length as well).
   for (u32 i0 = t - lane; i0 < nc; i0 += nt) {
     bool live = i0 + lane < nc;
     RangeCand c{};
@@ -1165,10 +1168,12 @@ __global__ void __launch_bounds__(128) k_range_finish(const __grid_constant__ Ra
       live = c.kind == 0 ? c.st >= *(volatile const ull*)&r->st_key
                          : key_of<4>(c.E) >= *(volatile const ull*)&r->e_key;
     }
-    for (u32 m = __ballot_sync(FULL, live); m; m &= m - 1) {
-      if (lane == (u32)__ffs(m) - 1) {
+    while (__any_sync(FULL, live)) {
+      const u32 same = __match_any_sync(FULL, live ? (ull)c.req : (1ull << 32) + lane);
+      if (live && lane == (u32)__ffs(same) - 1) {
         if (c.kind == 0) rec_offer_st(A.recs + c.req, c.st, c.seed);
         else rec_offer_e<4>(A.recs + c.req, c.E, c.seed);
+        live = false;
       }
       __syncwarp();
     }
