@@ -61,14 +61,14 @@ WINDOW_SAMPLE = 20000
 #   frontier: k_range on three-word values, at 2^60, k = 34: the pipes of a 2^36 launch, the dram
 #             bytes of a 2^40 launch (the 2.43 GB table about twice, however many blocks).
 NCU_CAPTURES = {
-    "block": {"src": "f2c27558ed8bb969", "dram_bytes": 4.679936e6 + 0.000768e6, "per": "launch",
-              "issue_slots_busy": 0.7515, "alu_pipe_busy": 0.6494, "kernel": "k_range (two words)"},
-    "frontier": {"src": "f2c27558ed8bb969", "dram_bytes": 5.180748e9 + 1.15155712e8, "per": "launch",
-                 "issue_slots_busy": 0.7961, "alu_pipe_busy": 0.7025, "kernel": "k_range (three words)"},
+    "block": {"src": "cb0235cfc9399013", "dram_bytes": 4.676096e6 + 0.001536e6, "per": "launch",
+              "issue_slots_busy": 0.7520, "alu_pipe_busy": 0.6506, "kernel": "k_range (two words)"},
+    "frontier": {"src": "cb0235cfc9399013", "dram_bytes": 5.18e9 + 1.2589e8, "per": "launch",
+                 "issue_slots_busy": 0.7975, "alu_pipe_busy": 0.7042, "kernel": "k_range (three words)"},
 }
 SHARED_KERNEL_SOURCES = ("common.cuh", "kernels.h", "tables.h", "tables.cu")
-KERNEL_SOURCES = {"block": ("range.cu",) + SHARED_KERNEL_SOURCES,
-                  "frontier": ("range.cu",) + SHARED_KERNEL_SOURCES}
+KERNEL_SOURCES = {"block": ("range.cu", "range_variants.h") + SHARED_KERNEL_SOURCES,
+                  "frontier": ("range.cu", "range_variants.h") + SHARED_KERNEL_SOURCES}
 # CPU sample of the block workload, the same for the reference arm's steps and
 # the cpu_baseline leg: 2^32 seeds at 2^40 + i 2^32 with the k = 24 sieve.
 CPU_SAMPLE_LOG2 = 32

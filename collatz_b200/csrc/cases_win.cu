@@ -237,10 +237,10 @@ __device__ __forceinline__ void exact_batch(const CasesArgs& A, uint2 e, bool ha
 // Lane state: v (0: idle; a fixed point of the look-ups that leaves the hash alone), n, the seed's
 // hash so far, the largest v in the limit's units and that limit, the look-ups left, the address of the
 // table for its next look-up; and the lane's next seed, so that a refill serves most lanes.
-// Bound by issue (77 % busy, the ALU 73 %): 19.7 warp instructions per seed against 49.7 with
+// Bound by issue (77 % busy, the ALU 75 %): 18.8 warp instructions per seed against 49.7 with
 // the runs counted in 64-bit pairs; a seed takes about six look-ups, so that half the
-// instructions hand seeds to lanes.  555 M seeds of one line: 21.7 -> 9.6 ms, 2048 lines:
-// 14.2 -> 6.5 ms.  Groups of 3 look-ups 9.9 ms, of 2 10.6; a refill at 26 lanes 9.7; without
+// instructions hand seeds to lanes.  555.7 M seeds of one line (27 10 8 183 0 0): 28.6 -> 11.9 ms,
+// 2048 lines: 14.2 -> 6.5 ms.  Groups of 3 look-ups 9.9 ms, of 2 10.6; a refill at 26 lanes 9.7; without
 // the next seed in the lane 10.1; 24 warps with 80 registers 10.1.
 template <bool MULTI, u32 UNIT>
 __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_constant__ CasesArgs A) {

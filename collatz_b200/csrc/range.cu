@@ -39,7 +39,7 @@
 // seeds at a time take their windows again from the start, with four words and a peak per
 // window (screen).  What may still change an output then, and every seed below 2^16, is
 // run one run pair at a time for the exact stopping time and excursion (exact_seeds):
-// 37 000 of the 7 million queued ones in 2^38 seeds.  A value that could leave 2^128 sends the
+// some 55 000 of the 3.2 million queued ones in 2^38 seeds.  A value that could leave 2^128 sends the
 // seed to the widen list, re-run with 6 and then 8 limbs.  A request whose maxima are still zero
 // gets a head start from a run's first seeds (scout).
 //

@@ -64,9 +64,8 @@ constexpr uint64_t TRAJ_BYTES_PER_SEED = 128;
 constexpr uint32_t MAX_ACTIVE_LIMIT = 4096;
 constexpr uint32_t MAX_BATCH_SEEDS = 1u << 22;
 // Staging reserved per admitted request for a slice's work list: a request
-// lowers to a dense part, up to 5 class segments for each partial block and
-// up to 45 (9 residues of q mod 9 x 5 kept classes) for the whole blocks in
-// between; more is allocated on demand.
+// lowers to a dense part, 5 class segments for each partial block (9 without the
+// mod-9 sieve) and 9 for the whole blocks in between; more is allocated on demand.
 constexpr size_t SEGS_PER_REQ = 64;
 
 // host-time buckets of the worker threads

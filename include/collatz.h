@@ -263,7 +263,8 @@ int collatz_verify_range(collatz_ctx *ctx, const collatz_range *r, collatz_range
 int collatz_verify_batch(collatz_ctx *ctx, const collatz_range *r, uint32_t n, collatz_range_result *out);
 
 /* Device-resident form for timing: a plan holds the lowered work list on
- * the device and a captured CUDA graph (reset, kernel, widening passes). */
+ * the device and a captured CUDA graph (reset, range kernel, candidates and wide
+ * seeds, copy back). */
 typedef struct collatz_plan collatz_plan;
 int collatz_plan_create(collatz_ctx *ctx, const collatz_range *r, uint32_t n, collatz_plan **out);
 int collatz_plan_launch(collatz_plan *p);   /* enqueue on the context stream, no sync */
@@ -366,8 +367,8 @@ int collatz_server_stop(collatz_server *s);
  *     refill thresholds).  0 to 5 run with 24 warps per block when a launch has
  *     few rows and with 32 otherwise; 6 and 7 are 0 with 32 and with 24;
  *   COLLATZ_MODE_RANGE64_BITS: the width -- launches whose seeds all have at
- *     most this many bits (0..52; those above 48 count as 48) keep values in
- *     two words, the others in three or four (0: never two).
+ *     most this many bits (0..48) keep values in two words, the others in three
+ *     or four (0: never two).
  * collatz_variant_count gives the number of choices (0..count-1). */
 #define COLLATZ_MODE_CASES 0
 #define COLLATZ_MODE_RANGE 1
