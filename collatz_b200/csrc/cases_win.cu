@@ -242,6 +242,7 @@ __device__ __forceinline__ void exact_batch(const CasesArgs& A, uint2 e, bool ha
 // instructions hand seeds to lanes.  555.7 M seeds of one line (27 10 8 183 0 0): 28.6 -> 11.9 ms,
 // 2048 lines: 14.2 -> 6.5 ms.  Groups of 3 look-ups 9.9 ms, of 2 10.6; a refill at 26 lanes 9.7; without
 // the next seed in the lane 10.1; 24 warps with 80 registers 10.1.
+// UNIT: the limits' unit, or 0 for A.unit.
 template <bool MULTI, u32 UNIT>
 __global__ void __launch_bounds__(WWARPS * 32, 1) k_cases_win(const __grid_constant__ CasesArgs A) {
   CwShared& S = *reinterpret_cast<CwShared*>(cw_smem);
